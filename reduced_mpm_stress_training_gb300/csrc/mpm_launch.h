@@ -26,8 +26,7 @@ cudaError_t launch_keys(const Ctx &cx);
 cudaError_t launch_sort(const Ctx &cx);
 
 // transfer stages (mpm_substep.cu)
-// partials / blk_index non-null: the ordered mode (see launch_p2g_ordered)
-cudaError_t launch_p2g(const Ctx &cx, float dt, float4 *partials = nullptr, int *blk_index = nullptr);
+cudaError_t launch_p2g(const Ctx &cx, float dt);
 // P2G whose sums do not depend on the order in which warps run (mpm_ordered.cu):
 // each cell's particles in uid order, per-block tiles to `scratch`, summed per
 // node in a fixed order into grid_acc.  scratch: ordered_scratch_bytes

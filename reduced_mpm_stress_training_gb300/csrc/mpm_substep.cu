@@ -6,11 +6,11 @@
 // one grid block have all their 3x3x3 stencils in the 6x6x6 node tile
 // anchored at that block.
 //
-//   p2g  -- one warp per non-empty block: per-cell runs of particles summed
-//           in registers and added to a warp-private tile in shared memory,
-//           each non-zero node flushed with ONE float4 atomicAdd to global
-//           memory, and the 8 grid blocks the tile covers registered in the
-//           active-block list.
+//   p2g  -- one CTA per non-empty block, a warp per x-slab: lanes are stencil
+//           nodes, per-cell runs of particles summed in registers and added
+//           to private slab tiles in shared memory, each non-zero node
+//           flushed with ONE float4 atomicAdd to global memory, and the 8
+//           grid blocks the tile covers registered in the active-block list.
 //   grid -- one thread per node of each active block: momentum/mass +
 //           gravity, colliders in registration order; clears the block
 //           flag.  (The accumulator is zeroed by the next substep's
@@ -32,354 +32,254 @@ namespace mpm {
 // P2G: p2g_apic_stress_given, engine_stress/mpm_utils.py:190-227
 //   grid_v_in += (w m)(v + C dpos) + dt (-vol tau) grad w,  grid_m += w m
 //
-// One warp per non-empty grid block, with a warp-private 6x6x6 node tile in
-// shared memory and no floating-point atomics in the particle loop.  The
-// sort delivers the block's particles ordered by cell with each cell's range
-// (cell_start .. cell_cursor).  Particles of one cell share their 27 stencil
-// nodes, so a lane takes a run of consecutive particles of one cell, sums
-// their contributions in registers (27 nodes x 4 = 108 accumulators) and
-// adds them to the tile once: the shared-memory read-modify-writes drop
-// from one per particle and node to one per run and node.  A round gives
-// each lane a run of the same length L from a DISTINCT cell, whose stencils
-// hit distinct nodes for every node offset -- the tile updates are
-// race-free.  The cells are chosen longest-remaining first (every cell with
-// at least t particles left, t the smallest threshold that leaves at most 32
-// such cells, filled up to 32 with cells that have t - 1 left: Hu's list
-// schedule for chains), and L is the fewest particles any chosen cell has
-// left, at most kRunMax, so no lane idles inside a round.  Each lane streams
-// its run's 128-byte records into shared memory with cp.async one particle
-// ahead.  The tile is flushed with one
-// float4 atomicAdd per non-zero node into the global grid.
+// One CTA of four warps per non-empty grid block.  The sort delivers the
+// block's particles ordered by cell (x slowest), so the particles of the four
+// cells-thick x-slabs are four contiguous ranges: warp w takes the slab with
+// local x = w, whose stencils cover three node planes.
 //
-// Tile layout: rows of 6 nodes along z padded to 8 slots and rotated by
-// 4 (y & 1), so a node's 16-byte bank group is (z + 4 (y & 1)) mod 8: the 8
-// lanes of a quarter-warp (one 128-bit shared access phase) holding two
-// y-adjacent rows of 4 cells hit 8 distinct bank groups for every offset.
+// A warp takes 32 of its particles at a time.  Each lane loads one record and
+// reduces it to the 25 numbers the scatter needs, in shared memory.  Then
+// three groups of nine lanes take a third of the 32 each: a group's lanes are
+// the nine (x, y) node offsets of the stencil, and each lane sums its three
+// z nodes (12 accumulators) over the group's consecutive particles until the
+// cell changes, when it adds them to the group's own slab tile (plain
+// read-modify-writes of distinct nodes, no atomics).  At the block's end the
+// CTA sums the tiles that cover each node of the 6x6x6 tile and issues one
+// float4 atomicAdd per non-zero node.
+//
+// What it replaces: one warp per block with a whole stencil (108 accumulators)
+// per lane, which fit eight warps on an SM at a third of the issue rate.  Here
+// 24 warps fit and a block's latency is a quarter; the limit is shared-memory
+// bandwidth (the 25 numbers are read by nine lanes each).  Measured per launch:
+// 19.0 -> 8 us on 4,096 particles, 90 -> 79 us on the 1M column.
 // ---------------------------------------------------------------------------
-constexpr int kP2GWarps = 1;  // one warp per CTA: the hardware balances unequal blocks
-constexpr int kRunMax = 4;     // most particles of one cell a lane takes per round
-constexpr int kP2GQuads = 8;   // record quads P2G reads (q0-q7, 128 B)
-constexpr int kRowSlots = 8;
-constexpr int kP2GSlots = kTile * kTile * kRowSlots;
+constexpr int kP2GWarps = 4;                  // one per x-slab of the block
+constexpr int kP2GQuads = 8;                  // record quads P2G reads (q0-q7, 128 B)
+constexpr int kP2GGroups = 3;                 // groups of nine lanes
+constexpr int kP2GPay = 7;                    // float4 of a particle's scatter data
+constexpr int kSlabPlane = kTile * kTile + 1; // nodes of a plane, padded: the rows of a stencil's
+                                              // nine lanes fall on (almost) distinct bank groups
+constexpr int kSlabNodes = 3 * kSlabPlane;
 
-__device__ __forceinline__ int p2g_slot(int x, int y, int z) {
-    return (x * kTile + y) * kRowSlots + ((z + 4 * (y & 1)) & 7);
-}
-
-struct P2GWarpSmem {
-    float4 tile[kP2GSlots];
-    float4 rec[2][kP2GQuads][32];  // each lane's current and next record
-    int4 seg[32];                  // the round's runs: first sorted position, cell
+struct P2GSmem {
+    float4 tile[kP2GWarps][kP2GGroups][kSlabNodes];
+    float4 pay[kP2GWarps][kP2GPay][32];
+    int used[kP2GWarps];  // the warp's slab holds particles
 };
 
-struct P2GParticle {
-    Weights W;
-    int lx, ly, lz;
-    float m;
-    float a0[3];  // v - C fx dx
-    float Cd[9];  // C dx
-    float T[9];   // -dt vol inv_dx tau
-};
-
+// one particle's scatter data (see p2g_add): the offsets fx and mass; v - C fx dx and
+// the cell within the block; C dx; -dt vol inv_dx tau.  False: not inside this block.
 __device__ __forceinline__ bool p2g_load(const MpmScene &S, const float4 (&q)[kP2GQuads], int bx, int by,
-                                         int bz, float dt, P2GParticle &P) {
+                                         int bz, float dt, float4 (&o)[kP2GPay]) {
     // record quads 0-7: x0 m | vol .. | u v.x | v.yz C0 C1 | C2-5 | C6-8 tau0 | tau1-4 | tau5-8
     const float4 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4], q5 = q[5], q6 = q[6], q7 = q[7];
     const float x0[3] = {q0.x, q0.y, q0.z}, u[3] = {q2.x, q2.y, q2.z};
-    float gp[3];
+    float fx[3];
     int base[3];
     bool ok = true;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        gp[d] = grid_coord(x0[d], u[d], S.inv_dx);
-        ok &= stencil_base(gp[d], S.n_grid, base[d]);
+        const float gp = grid_coord(x0[d], u[d], S.inv_dx);
+        ok &= stencil_base(gp, S.n_grid, base[d]);
+        fx[d] = __fsub_rn(gp, (float)base[d]);
     }
-    P.lx = base[0] - 4 * bx;
-    P.ly = base[1] - 4 * by;
-    P.lz = base[2] - 4 * bz;
-    ok &= (unsigned)P.lx < 4u && (unsigned)P.ly < 4u && (unsigned)P.lz < 4u;
-    if (!ok) return false;
-    make_weights(gp, base, P.W);
-    P.m = q0.w;
-    const float vol = q1.x;
+    const int lx = base[0] - 4 * bx, ly = base[1] - 4 * by, lz = base[2] - 4 * bz;
+    ok &= (unsigned)lx < 4u && (unsigned)ly < 4u && (unsigned)lz < 4u;
     const float dx = S.dx;
     const float v[3] = {q2.w, q3.x, q3.y};
     const float Cm[9] = {q3.z, q3.w, q4.x, q4.y, q4.z, q4.w, q5.x, q5.y, q5.z};
     const float tau[9] = {q5.w, q6.x, q6.y, q6.z, q6.w, q7.x, q7.y, q7.z, q7.w};
-    const float tscale = -vol * dt * S.inv_dx;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) P.T[k] = tau[k] * tscale;
+    const float ts = -q1.x * dt * S.inv_dx;  // -vol dt / dx
+    float a0[3];
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-        const float cf = Cm[r * 3 + 0] * P.W.fx[0] + Cm[r * 3 + 1] * P.W.fx[1] + Cm[r * 3 + 2] * P.W.fx[2];
-        P.a0[r] = v[r] - cf * dx;
+        const float cf = Cm[r * 3 + 0] * fx[0] + Cm[r * 3 + 1] * fx[1] + Cm[r * 3 + 2] * fx[2];
+        a0[r] = v[r] - cf * dx;
     }
-#pragma unroll
-    for (int k = 0; k < 9; ++k) P.Cd[k] = Cm[k] * dx;
-    return true;
+    o[0] = make_float4(fx[0], fx[1], fx[2], q0.w);
+    o[1] = make_float4(a0[0], a0[1], a0[2], __int_as_float((lx << 4) | (ly << 2) | lz));
+    o[2] = make_float4(Cm[0] * dx, Cm[3] * dx, Cm[6] * dx, Cm[8] * dx);
+    o[3] = make_float4(Cm[1] * dx, Cm[4] * dx, Cm[7] * dx, tau[8] * ts);
+    o[4] = make_float4(Cm[2] * dx, Cm[5] * dx, tau[0] * ts, tau[3] * ts);
+    o[5] = make_float4(tau[6] * ts, tau[1] * ts, tau[4] * ts, tau[7] * ts);
+    o[6] = make_float4(tau[2] * ts, tau[5] * ts, 0.0f, 0.0f);
+    return ok;
 }
 
-// add one particle's 27 node contributions to the lane's accumulators
-// (x, y packed in axy, z and mass in azw: Blackwell's two-wide FP32 FMA).
-// Per (i,j) the node value factors over k:
-//   add_r = wz_k A_r + k wz_k B_r + dwz_k D_r,  mass = pm wz_k
+// a lane's stencil offset (i, j): weight s (f - c)^2 + t and its derivative 2 s (f - c) per axis
+struct P2GLane {
+    float fi, fj, cx, sx, tx, cy, sy, ty;
+};
+__device__ __forceinline__ void p2g_axis(int i, float &c, float &s, float &t) {
+    c = i == 0 ? 1.5f : (i == 1 ? 1.0f : 0.5f);
+    s = i == 1 ? -1.0f : 0.5f;
+    t = i == 1 ? 0.75f : 0.0f;
+}
+
+// add one particle's contributions to the lane's three z nodes.  Per (i, j) the
+// node value factors over k:
+//   add_r = wz_k (A_r + k B_r) + dwz_k D_r,  mass = wz_k pm
 // with pm = wx_i wy_j m, A_r = pm (a0_r + i Cdx_r + j Cdy_r) + T_r0 dwx_i wy_j
 // + T_r1 wx_i dwy_j, B_r = pm Cdz_r, D_r = T_r2 wx_i wy_j.
-__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ void p2g_add(const P2GLane &L, const float4 (&o)[kP2GPay], float (&acc)[3][4]) {
+    const float dxi = o[0].x - L.cx, dyj = o[0].y - L.cy;
+    const float ex = L.sx * dxi, ey = L.sy * dyj;
+    const float wx = fmaf(ex, dxi, L.tx), wy = fmaf(ey, dyj, L.ty);
+    const float za = o[0].z - 1.5f, zb = o[0].z - 1.0f, zc = o[0].z - 0.5f;
+    const float w[3] = {0.5f * za * za, fmaf(-zb, zb, 0.75f), 0.5f * zc * zc};
+    const float dw[3] = {za, -2.0f * zb, zc};
+    const float p1 = 2.0f * ex * wy, p2 = 2.0f * ey * wx, p3 = wx * wy, pm = p3 * o[0].w;
+    const float a0[3] = {o[1].x, o[1].y, o[1].z};
+    const float cdx[3] = {o[2].x, o[2].y, o[2].z}, cdy[3] = {o[3].x, o[3].y, o[3].z};
+    const float cdz[3] = {o[4].x, o[4].y, o[2].w};
+    const float t0[3] = {o[4].z, o[4].w, o[5].x}, t1[3] = {o[5].y, o[5].z, o[5].w};
+    const float t2[3] = {o[6].x, o[6].y, o[3].w};
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const float a = fmaf(L.fi, cdx[r], fmaf(L.fj, cdy[r], a0[r]));
+        const float A0 = fmaf(pm, a, fmaf(t0[r], p1, t1[r] * p2));
+        const float A1 = fmaf(pm, cdz[r], A0), A2 = fmaf(pm, cdz[r], A1);
+        const float D = t2[r] * p3;
+        acc[0][r] = fmaf(w[0], A0, fmaf(dw[0], D, acc[0][r]));
+        acc[1][r] = fmaf(w[1], A1, fmaf(dw[1], D, acc[1][r]));
+        acc[2][r] = fmaf(w[2], A2, fmaf(dw[2], D, acc[2][r]));
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) acc[k][3] = fmaf(w[k], pm, acc[k][3]);
+}
 
-__device__ __forceinline__ void p2g_accumulate(const P2GParticle &P, float2 (&axy)[27], float2 (&azw)[27]) {
-    const float2 a0 = f2(P.a0[0], P.a0[1]);
-    const float2 cdx = f2(P.Cd[0], P.Cd[3]), cdy = f2(P.Cd[1], P.Cd[4]), cdz = f2(P.Cd[2], P.Cd[5]);
-    const float2 t0 = f2(P.T[0], P.T[3]), t1 = f2(P.T[1], P.T[4]), t2 = f2(P.T[2], P.T[5]);
+// add a lane's sums of one cell (its y, z within the slab) to its three nodes of
+// the group's tile and clear them.  The group's lanes write distinct nodes here,
+// but an earlier flush may have been another lane's: order the group first.
+__device__ __forceinline__ void p2g_flush(float4 *mytile, int cell, unsigned gmask, float (&acc)[3][4]) {
+    float4 *t = mytile + (cell >> 2) * kTile + (cell & 3);
+    __syncwarp(gmask);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const float p1 = P.W.dw[0][i] * P.W.w[1][j];
-            const float p2 = P.W.w[0][i] * P.W.dw[1][j];
-            const float p3 = P.W.w[0][i] * P.W.w[1][j];
-            const float pm = p3 * P.m;
-            float2 aij = a0;
-            if (i > 0) aij = __ffma2_rn(f2((float)i, (float)i), cdx, aij);
-            if (j > 0) aij = __ffma2_rn(f2((float)j, (float)j), cdy, aij);
-            const float2 A = __ffma2_rn(f2(pm, pm), aij, __ffma2_rn(t0, f2(p1, p1), __fmul2_rn(t1, f2(p2, p2))));
-            const float2 B = __fmul2_rn(f2(pm, pm), cdz);
-            const float2 D = __fmul2_rn(t2, f2(p3, p3));
-            const float az = P.a0[2] + (float)i * P.Cd[6] + (float)j * P.Cd[7];
-            const float Az = pm * az + P.T[6] * p1 + P.T[7] * p2;
-            const float Bz = pm * P.Cd[8];
-            const float Dz = P.T[8] * p3;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float wz = P.W.w[2][k], dwz = P.W.dw[2][k];
-                float2 &xy = axy[(i * 3 + j) * 3 + k];
-                float2 &zw = azw[(i * 3 + j) * 3 + k];
-                xy = __ffma2_rn(f2(wz, wz), A, xy);
-                zw = __ffma2_rn(f2(wz, wz), f2(Az, pm), zw);
-                xy = __ffma2_rn(f2(dwz, dwz), D, xy);
-                zw.x = fmaf(dwz, Dz, zw.x);
-                if (k > 0) {
-                    const float kwz = k == 1 ? wz : 2.0f * wz;
-                    xy = __ffma2_rn(f2(kwz, kwz), B, xy);
-                    zw.x = fmaf(kwz, Bz, zw.x);
-                }
-            }
-        }
+    for (int k = 0; k < 3; ++k) {
+        float4 v = t[k];
+        v.x += acc[k][0];
+        v.y += acc[k][1];
+        v.z += acc[k][2];
+        v.w += acc[k][3];
+        t[k] = v;
+        acc[k][0] = acc[k][1] = acc[k][2] = acc[k][3] = 0.0f;
     }
 }
 
-// add a segment's accumulated nodes into the tile (read-modify-write; the
-// lanes of `mask` hold distinct cells)
-__device__ __forceinline__ void p2g_flush(const float2 (&axy)[27], const float2 (&azw)[27], int lx, int ly,
-                                          int lz, float4 *tile, unsigned mask) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                float4 *t = tile + p2g_slot(lx + i, ly + j, lz + k);
-                const int n = (i * 3 + j) * 3 + k;
-                float4 o = *t;
-                o.x += axy[n].x;
-                o.y += axy[n].y;
-                o.z += azw[n].x;
-                o.w += azw[n].y;
-                *t = o;
-                __syncwarp(mask);
-            }
-}
-
-__device__ __forceinline__ void p2g_cp_async16(void *smem, const void *gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-
-// queue the copy of one record (slot >= 0) into the lane's buffer b
-__device__ __forceinline__ void p2g_prefetch(P2GWarpSmem &sm, const PState &st, int slot, int b, int lane, int n) {
-    if (slot >= 0 && slot < n) {
-#pragma unroll
-        for (int q = 0; q < kP2GQuads; ++q) p2g_cp_async16(&sm.rec[b][q][lane], recq(st, slot, q));
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-
-// Choose the next round of a block: up to 32 distinct cells, longest
-// remaining first, each giving its next L particles.  Lane `lane` owns cells
-// lane and lane + 32 (remaining counts rem0/rem1, next positions pos0/pos1).
-// Returns false when the block is done; else the lane's run (first sorted
-// position, cell, length len: L or 0) and the round length L.
-__device__ __forceinline__ bool p2g_next_round(int &rem0, int &rem1, int &pos0, int &pos1, int lane, unsigned lt,
-                                               int4 *seg, int &start, int &cell, int &len, int &L) {
-    const unsigned full = 0xffffffffu;
-    const int maxrem = __reduce_max_sync(full, max(rem0, rem1));
-    if (maxrem == 0) return false;
-    // smallest t >= 1 with at most 32 cells holding >= t particles
-    int lo = 1, hi = maxrem + 1;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        const int cnt = __popc(__ballot_sync(full, rem0 >= mid)) + __popc(__ballot_sync(full, rem1 >= mid));
-        if (cnt <= 32) hi = mid;
-        else lo = mid + 1;
-    }
-    const unsigned h0 = __ballot_sync(full, rem0 >= lo), h1 = __ballot_sync(full, rem1 >= lo);
-    const int need = 32 - __popc(h0) - __popc(h1);
-    const unsigned f0 = __ballot_sync(full, lo > 1 && rem0 == lo - 1);
-    const unsigned f1 = __ballot_sync(full, lo > 1 && rem1 == lo - 1);
-    const bool p0 = rem0 >= lo || (((f0 >> lane) & 1u) && __popc(f0 & lt) < need);
-    const bool p1 = rem1 >= lo || (((f1 >> lane) & 1u) && __popc(f0) + __popc(f1 & lt) < need);
-    const unsigned b0 = __ballot_sync(full, p0), b1 = __ballot_sync(full, p1);
-    // every chosen cell gives its next L particles, L = the fewest any of them has left
-    const unsigned least =
-        __reduce_min_sync(full, min(p0 ? (unsigned)rem0 : 0xffffffffu, p1 ? (unsigned)rem1 : 0xffffffffu));
-    L = min((int)least, kRunMax);
-    if (p0) {
-        seg[__popc(b0 & lt)] = make_int4(pos0, lane, 0, 0);
-        pos0 += L;
-        rem0 -= L;
-    }
-    if (p1) {
-        seg[__popc(b0) + __popc(b1 & lt)] = make_int4(pos1, lane + 32, 0, 0);
-        pos1 += L;
-        rem1 -= L;
-    }
-    const int tot = __popc(b0) + __popc(b1);
-    __syncwarp();
-    const int4 mine = lane < tot ? seg[lane] : make_int4(0, 0, 0, 0);
-    __syncwarp();  // seg[] is rewritten by the next call
-    start = mine.x;
-    cell = mine.y;
-    len = lane < tot ? L : 0;
-    return true;
-}
-
-// partials == nullptr: the tile is flushed with float4 atomics into grid_acc.
-// Otherwise (the ordered mode of mpm_p2g_ordered) the whole 6x6x6 tile of
-// work-list entry bi goes to partials[bi] and blk_index[block] = bi; the
-// gather kernel then sums the <= 8 tiles covering each node in a fixed order.
-__global__ void __launch_bounds__(kP2GWarps * 32, 2) p2g_kernel(const MpmScene *__restrict__ scenes,
+__global__ void __launch_bounds__(kP2GWarps * 32, 6) p2g_kernel(const MpmScene *__restrict__ scenes,
                                                                 int n_scenes, PState st, Ws ws, float dt,
-                                                                int *status, float4 *partials,
-                                                                int *blk_index) {
+                                                                int *status) {
     extern __shared__ __align__(16) unsigned char p2g_smem_raw[];
-    P2GWarpSmem *smem = reinterpret_cast<P2GWarpSmem *>(p2g_smem_raw);
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    P2GWarpSmem &sm = smem[threadIdx.x >> 5];
+    P2GSmem &sm = *reinterpret_cast<P2GSmem *>(p2g_smem_raw);
+    const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int group = lane / 9;                    // 0-2; lanes 27-31 only load
+    const int ij = lane - 9 * group;
+    const int li = ij / 3, lj = ij - 3 * li;
+    P2GLane L;
+    L.fi = (float)li;
+    L.fj = (float)lj;
+    p2g_axis(li, L.cx, L.sx, L.tx);
+    p2g_axis(lj, L.cy, L.sy, L.ty);
+    const unsigned gmask = 0x1ffu << (9 * (group < kP2GGroups ? group : 0));
+    float4 *mytile = sm.tile[warp][group < kP2GGroups ? group : 0] + li * kSlabPlane + lj * kTile;
     const int nblk = *ws.n_blocks;
-    for (int bi = blockIdx.x * kP2GWarps + (int)(threadIdx.x >> 5); bi < nblk;
-         bi += gridDim.x * kP2GWarps) {
+    for (int bi = blockIdx.x; bi < nblk; bi += gridDim.x) {
         const int4 be = ws.blocks[bi];
         if ((unsigned)be.x >= (unsigned)(ws.nbk - 1) || (unsigned)be.w >= (unsigned)n_scenes) {
-            // a damaged work list: skip, never index with it
-            if (lane == 0) atomicOr(status, MPM_ST_INTERNAL);
+            // a damaged work list: skip, never index with it (uniform over the CTA)
+            if (tid == 0) atomicOr(status, MPM_ST_INTERNAL);
             continue;
         }
-        // by value: the compiler loads the few fields P2G uses once per block into
-        // registers (measured 1 us per launch faster than reading them through a reference)
-        const MpmScene S = scenes[be.w];
+        const MpmScene &S = scenes[be.w];
         int bx, by, bz;
         chunk_block(S, be.x, bx, by, bz);
-        for (int i = lane; i < kP2GSlots; i += 32) sm.tile[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        // cell ranges of this block: lane owns cells lane and lane + 32
-        const int64_t cb = (int64_t)be.x * 64;
-        const int s0 = ws.cell_start[cb + lane], s1 = ws.cell_start[cb + lane + 32];
-        const int c0 = max(0, ws.cell_cursor[cb + lane] - s0);
-        const int c1 = max(0, ws.cell_cursor[cb + lane + 32] - s1);
-        // Rounds are software-pipelined: while round A is summed, round B is
-        // chosen and its order[] entries load, and A's last iteration already
-        // streams B's first records.
-        int rem0 = c0, rem1 = c1, pos0 = s0, pos1 = s1;
-        int startA, cellA, lenA, LA;
-        bool haveA = p2g_next_round(rem0, rem1, pos0, pos1, lane, lt, sm.seg, startA, cellA, lenA, LA);
-        int slA[kRunMax];
+        // this warp's slab: cells 16 warp .. 16 warp + 15 of the block
+        const int64_t cb = (int64_t)be.x * 64 + 16 * warp;
+        const int s0 = ws.cell_start[cb], s1 = ws.cell_cursor[cb + 15];
+        bool bad = s0 < 0 || s1 > ws.n;
+        const int end = bad ? s0 : s1;
+        if (lane == 0) sm.used[warp] = end > s0;
+        if (end > s0)
+            for (int i = lane; i < kP2GGroups * kSlabNodes; i += 32)
+                (&sm.tile[warp][0][0])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        float acc[3][4];
 #pragma unroll
-        for (int t = 0; t < kRunMax; ++t) slA[t] = t < lenA && startA + t < ws.n ? ws.order[startA + t] : -1;
-        int buf = 0;
-        if (haveA) p2g_prefetch(sm, st, slA[0], 0, lane, ws.n);
-        bool bad = false;
-        while (haveA) {
-            int startB, cellB, lenB, LB;
-            const bool haveB = p2g_next_round(rem0, rem1, pos0, pos1, lane, lt, sm.seg, startB, cellB, lenB, LB);
-            int slB[kRunMax];
+        for (int k = 0; k < 3; ++k)
 #pragma unroll
-            for (int t = 0; t < kRunMax; ++t)
-                slB[t] = haveB && t < lenB && startB + t < ws.n ? ws.order[startB + t] : -1;
-            const int cx = cellA >> 4, cy = (cellA >> 2) & 3, cz = cellA & 3;
-            float2 axy[27], azw[27];
+            for (int r = 0; r < 4; ++r) acc[k][r] = 0.0f;
+        int slot = s0 + lane < end ? ws.order[s0 + lane] : -1;
+        for (int p0 = s0; p0 < end; p0 += 32) {
+            const int cnt = min(32, end - p0);
+            __syncwarp();  // the previous batch is consumed (and the tile cleared)
+            if (lane < cnt) {
+                float4 o[kP2GPay];
+                bool ok = (unsigned)slot < (unsigned)ws.n;
+                if (ok) {
+                    float4 q[kP2GQuads];
 #pragma unroll
-            for (int k = 0; k < 27; ++k) {
-                axy[k] = make_float2(0.f, 0.f);
-                azw[k] = make_float2(0.f, 0.f);
+                    for (int k = 0; k < kP2GQuads; ++k) q[k] = ldrec(st, slot, k);
+                    ok = p2g_load(S, q, bx, by, bz, dt, o) && (__float_as_int(o[1].w) >> 4) == warp;
+                }
+                if (!ok) {  // contributes zeros
+                    bad = true;
+#pragma unroll
+                    for (int k = 0; k < kP2GPay; ++k) o[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int k = 0; k < kP2GPay; ++k) sm.pay[warp][k][lane] = o[k];
             }
+            const int pn = p0 + 32 + lane;
+            slot = pn < end ? ws.order[pn] : -1;  // the next batch's, while this one is summed
+            __syncwarp();
+            const int per = (cnt + kP2GGroups - 1) / kP2GGroups;
+            const int first = group * per, last = group < kP2GGroups ? min(cnt, first + per) : 0;
+            int cur = -1;  // the cell being summed
+            for (int p = first; p < last; ++p) {
+                float4 o[kP2GPay];
 #pragma unroll
-            for (int t = 0; t < kRunMax; ++t) {
-                if (t < LA) {  // warp-uniform
-                    // the next record (this run's, or the next round's first) streams in
-                    // while this one is summed
-                    int nxt = slB[0];
+                for (int k = 0; k < kP2GPay; ++k) o[k] = sm.pay[warp][k][p];
+                const int cell = __float_as_int(o[1].w) & 15;  // y, z within the slab
+                if (cell != cur && cur >= 0) p2g_flush(mytile, cur, gmask, acc);
+                cur = cell;
+                p2g_add(L, o, acc);
+            }
+            if (cur >= 0) p2g_flush(mytile, cur, gmask, acc);
+        }
+        if (bad) atomicOr(status, MPM_ST_INTERNAL);
+        __syncthreads();
+        // the block's 6x6x6 tile: node plane x is covered by the slabs x - 2 .. x
+        const int nb = S.n_blocks_axis;
+        for (int i = tid; i < kTileNodes; i += kP2GWarps * 32) {
+            const int tx = i / (kTile * kTile), yz = i - tx * (kTile * kTile);
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                    for (int u = 0; u + 1 < kRunMax; ++u)
-                        if (u == t && t + 1 < LA) nxt = slA[u + 1];
-                    p2g_prefetch(sm, st, nxt, buf ^ 1, lane, ws.n);
-                    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-                    if (t < lenA && slA[t] < 0) {
-                        bad = true;  // position or slot out of range: nothing was staged
-                    } else if (t < lenA) {
-                        float4 q[kP2GQuads];
+            for (int d = 0; d < 3; ++d) {
+                const int w = tx - d;
+                if (w < 0 || w >= kP2GWarps || !sm.used[w]) continue;
 #pragma unroll
-                        for (int qq = 0; qq < kP2GQuads; ++qq) q[qq] = sm.rec[buf][qq][lane];
-                        P2GParticle P;
-                        const bool ok =
-                            p2g_load(S, q, bx, by, bz, dt, P) && P.lx == cx && P.ly == cy && P.lz == cz;
-                        if (ok) p2g_accumulate(P, axy, azw);
-                        bad |= !ok;
-                    }
-                    buf ^= 1;
+                for (int g = 0; g < kP2GGroups; ++g) {
+                    const float4 v = sm.tile[w][g][d * kSlabPlane + yz];
+                    a.x += v.x;
+                    a.y += v.y;
+                    a.z += v.z;
+                    a.w += v.w;
                 }
             }
-            const unsigned fm = __ballot_sync(full, lenA > 0);
-            if (lenA > 0) p2g_flush(axy, azw, cx, cy, cz, sm.tile, fm);
-            __syncwarp();
-            haveA = haveB;
-            startA = startB;
-            cellA = cellB;
-            lenA = lenB;
-            LA = LB;
-#pragma unroll
-            for (int t = 0; t < kRunMax; ++t) slA[t] = slB[t];
-        }
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        if (bad) atomicOr(status, MPM_ST_INTERNAL);
-        const int nb = S.n_blocks_axis;
-        if (partials) {
-            // ordered mode: the whole tile to this entry's slot, in node order
-            float4 *dst = partials + (int64_t)bi * kTileNodes;
-            for (int i = lane; i < kTileNodes; i += 32)
-                dst[i] = sm.tile[p2g_slot(i / (kTile * kTile), (i / kTile) % kTile, i % kTile)];
-            if (lane == 0) blk_index[be.x] = bi;
-        }
-        // flush the tile: one float4 atomic per non-zero node
-        for (int i = lane; i < kP2GSlots && !partials; i += 32) {
-            const float4 a = sm.tile[i];
             if (a.x != 0.0f || a.y != 0.0f || a.z != 0.0f || a.w != 0.0f) {
-                const int tx = i / (kTile * kRowSlots), ty = (i / kRowSlots) % kTile;
-                const int tz = ((i & 7) - 4 * (ty & 1)) & 7;  // unused slots (tz 6, 7) stay zero
-                const int ix = 4 * bx + tx, iy = 4 * by + ty, iz = 4 * bz + tz;
+                const int ix = 4 * bx + tx, iy = 4 * by + yz / kTile, iz = 4 * bz + yz % kTile;
                 if (ix < S.n_grid && iy < S.n_grid && iz < S.n_grid)
                     atomicAdd(ws.grid_acc + node_addr(S.block_begin, nb, ix, iy, iz), a);
             }
         }
-        if (lane < 8) {
-            const int gx = bx + (lane >> 2), gy = by + ((lane >> 1) & 1), gz = bz + (lane & 1);
+        if (tid < 8) {
+            const int gx = bx + (tid >> 2), gy = by + ((tid >> 1) & 1), gz = bz + (tid & 1);
             if (gx < nb && gy < nb && gz < nb) {
                 const int gb = (int)(S.block_begin + ((int64_t)(gx * nb + gy) * nb + gz));
                 if (atomicExch(ws.block_flag + gb, 1) == 0)
                     ws.active_list[atomicAdd(ws.n_active, 1)] = gb;
             }
         }
-        __syncwarp();
+        __syncthreads();  // the tiles are read: the next block may clear them
     }
 }
 
@@ -770,26 +670,16 @@ static cudaError_t g2p_t(const Ctx &cx, float dt) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_p2g(const Ctx &cx, float dt, float4 *partials, int *blk_index) {
-    // more than the 48 KB of static shared memory: opt in once per device
-    static bool attr_set[64] = {false};
-    const int bytes = (int)(sizeof(P2GWarpSmem) * kP2GWarps);
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        e = cudaFuncSetAttribute(p2g_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) attr_set[dev] = true;
-    }
-    // up to 32 single-warp CTAs per SM, several times the resident ones: the
-    // rest start as others finish, which balances blocks of unequal size;
-    // warps loop over blocks when there are more blocks than warps
-    int64_t want = (cx.total_blocks + kP2GWarps - 1) / kP2GWarps;
-    int grid = (int)(want < (int64_t)cx.num_sms * 32 ? want : (int64_t)cx.num_sms * 32);
+cudaError_t launch_p2g(const Ctx &cx, float dt) {
+    const int bytes = (int)sizeof(P2GSmem);
+    static_assert(sizeof(P2GSmem) <= 48 * 1024, "static shared-memory limit");
+    // up to 24 CTAs per SM, several times the resident ones: the rest start as
+    // others finish, which balances blocks of unequal size; CTAs loop over
+    // blocks when there are more blocks than CTAs
+    int grid = (int)(cx.total_blocks < (int64_t)cx.num_sms * 24 ? cx.total_blocks : (int64_t)cx.num_sms * 24);
     if (grid < 1) grid = 1;
     p2g_kernel<<<grid, kP2GWarps * 32, bytes, cx.stream>>>(cx.scenes, cx.n_scenes, cx.st, cx.ws, dt,
-                                                           cx.status, partials, blk_index);
+                                                           cx.status);
     return cudaGetLastError();
 }
 

@@ -1,0 +1,62 @@
+"""P2G at the edges of its work split, against the float32 oracle: particle
+counts around a warp's batch of 32 and its three groups, in one cell, in one
+x-slab of a grid block, in one block and over blocks that the grid cuts off;
+and blocks whose slabs are empty.
+
+Tolerance: the per-substep bar of the parity tests, 1e-5 relative L2 on grid
+mass and momentum (a node sums at most a few hundred rounded terms, about
+1e-6 of their norm in float32).
+"""
+import numpy as np
+import pytest
+import torch
+
+from reduced_mpm_stress_training_gb300 import scenarios as S
+
+from helpers import gpu_sim, oracle_sim, rel
+
+pytestmark = pytest.mark.gpu
+
+N_GRID = 18  # the last 4x4x4 block of an axis holds two node planes
+TOL = 1e-5
+
+
+def _cells(where, n, rng):
+    """Base cells (n, 3): block (1, 2, 1) spans cells 4-7, 8-11, 4-7."""
+    lo, hi = {"cell": ((6, 9, 5), (7, 10, 6)), "slab": ((5, 8, 4), (6, 12, 8)), "block": ((4, 8, 4), (8, 12, 8)),
+              "two_slabs": ((4, 8, 4), (8, 12, 8)), "edge": ((13, 13, 13), (16, 16, 16))}[where]
+    c = np.stack([rng.integers(lo[d], hi[d], n) for d in range(3)], 1)
+    if where == "two_slabs":  # slabs 1 and 2 stay empty
+        c[:, 0] = np.where(c[:, 0] < 6, 4, 7)
+    return c
+
+
+@pytest.mark.parametrize("where", ["cell", "slab", "block", "two_slabs", "edge"])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 31, 32, 33, 63, 64, 65, 97, 300])
+def test_p2g_split_matches_oracle(cuda, where, n):
+    rng = np.random.default_rng(1000 + n)
+    sc = S.small_column(n, N_GRID)
+    # x / dx = base + 0.5 + [0.01, 0.99): clear of the cell borders
+    x0 = ((_cells(where, n, rng) + 0.5 + rng.uniform(0.01, 0.99, (n, 3))) / N_GRID).astype(np.float32)
+    v = rng.normal(size=(n, 3)).astype(np.float32)
+    Cm = (0.5 * rng.normal(size=(n, 9))).astype(np.float32)
+    tau = (1e3 * rng.normal(size=(n, 9))).astype(np.float32)
+    vol = np.full(n, 1e-5, np.float32)
+    mass = (rng.uniform(1.0, 2.0, n) * 1e-2).astype(np.float32)
+    sim = gpu_sim(sc, x0=x0, v0=v, vol=vol, mass=mass)
+    sim.load_C_from_tensor(torch.from_numpy(Cm))
+    sim.load_uvstress_from_tensor(torch.zeros(n, 3), torch.from_numpy(v), torch.from_numpy(tau))
+    ref = oracle_sim(sc, x0=x0, v0=v, vol=vol, mass=mass)
+    ref.C[:] = Cm
+    ref.stress[:] = tau
+    e = sim.engine
+    for _ in range(2):  # the second time the previous grid has to be cleared
+        e.stage("sort")
+        e.stage("p2g", dt=sc.dt)
+        gm, gvin, _ = e.export_grid(0)
+        e.buf.keys_valid = 0
+        ref.stage_p2g(sc.dt)
+        assert rel(gm.cpu().numpy(), ref.grid_m) < TOL
+        assert rel(gvin.cpu().numpy(), ref.grid_v_in) < TOL
+        e.stage("grid", time=0.0, dt=sc.dt)
+    assert e.status() == 0
