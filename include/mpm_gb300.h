@@ -124,7 +124,8 @@ typedef struct MpmPlan {
 } MpmPlan; /* 56 bytes */
 
 /* Caller-owned device buffers plus the host-side control the library keeps
- * between calls.  All pointers are device pointers (256-byte aligned). */
+ * between calls.  All pointers are device pointers (256-byte aligned; calls
+ * refuse state buffers that are not at least 32-byte aligned). */
 typedef struct MpmBuffers {
     void *state[2];   /* two particle-state buffers, plan.state_bytes each      */
     void *workspace;  /* plan.workspace_bytes                                  */
@@ -238,7 +239,9 @@ int mpm_export_frame(MpmBuffers *b, float *out, void *stream);
 int mpm_p2g2p(MpmBuffers *b, float time, float dt, void *stream);
 
 /* The substep's stages, for callers that interleave their own work and for
- * per-stage checks.  mpm_p2g2p == sort, p2g, grid_update, g2p. */
+ * per-stage checks.  mpm_p2g2p == sort, p2g, grid_update, g2p up to float32
+ * rounding: it runs its own compilation of the last stage, while mpm_g2p keeps
+ * one whose float32 results stay the same bit for bit. */
 int mpm_sort(MpmBuffers *b, void *stream); /* block keys, counting sort, re-sort */
 int mpm_p2g(MpmBuffers *b, float dt, void *stream); /* mpm_utils.py:190-227 */
 int mpm_grid_update(MpmBuffers *b, float time, float dt, void *stream); /* :229-237 + colliders */

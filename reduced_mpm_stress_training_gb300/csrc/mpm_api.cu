@@ -101,15 +101,13 @@ int64_t mpm::substep_workspace_bytes(const MpmPlan &p) { return ws_layout(p).sta
 
 namespace {
 
-// [quads 0-3 of every slot][quads 4-7][quads 8-9][cell keys]; stride is a
-// multiple of 64 slots, so every array starts 4 KB-aligned
+// [quad pairs 0-1, 2-3, 4-5, 6-7, 8-9 of every slot][cell keys]; stride is a
+// multiple of 64 slots, so every array starts 2 KB-aligned
 mpm::PState state_view(void *base, int64_t stride) {
     mpm::PState s;
     char *p = static_cast<char *>(base);
     s.stride = stride;
-    s.a = reinterpret_cast<float4 *>(p);
-    s.b = reinterpret_cast<float4 *>(p + stride * 64);
-    s.f = reinterpret_cast<float4 *>(p + stride * 128);
+    s.q = reinterpret_cast<float4 *>(p);
     s.key = reinterpret_cast<int *>(p + stride * mpm::kRecWords * 4);
     return s;
 }
@@ -156,8 +154,10 @@ mpm::Ctx make_ctx(const MpmBuffers *b, void *stream, int which) {
     return cx;
 }
 
+// (the state's records move in 32-byte accesses)
 bool buffers_ok(const MpmBuffers *b) {
-    return b && b->state[0] && b->state[1] && b->workspace && b->scenes && b->status &&
+    return b && b->state[0] && b->state[1] &&
+           !((reinterpret_cast<uintptr_t>(b->state[0]) | reinterpret_cast<uintptr_t>(b->state[1])) & 31) && b->workspace && b->scenes && b->status &&
            b->plan.n_scenes >= 1 && (b->cur == 0 || b->cur == 1);
 }
 
@@ -432,7 +432,7 @@ int mpm_grid_update(MpmBuffers *b, float time, float dt, void *stream) {
 int mpm_g2p(MpmBuffers *b, float dt, void *stream) {
     NvtxRange nvtx_("mpm_g2p");
     if (!buffers_ok(b)) return MPM_ERR_ARG;
-    MPM_CHECK(mpm::launch_g2p(make_ctx(b, stream, b->cur), dt));
+    MPM_CHECK(mpm::launch_g2p(make_ctx(b, stream, b->cur), dt, mpm::G2PForm::kPinned));
     b->cur ^= 1;  // G2P wrote the sorted, updated records into the other buffer
     b->substep += 1;
     return MPM_OK;
@@ -465,7 +465,10 @@ int mpm_p2g2p(MpmBuffers *b, float time, float dt, void *stream) {
     if (r) return r;
     if ((r = mpm_p2g(b, dt, stream))) return r;
     if ((r = mpm_grid_update(b, time, dt, stream))) return r;
-    return mpm_g2p(b, dt, stream);
+    MPM_CHECK(mpm::launch_g2p(make_ctx(b, stream, b->cur), dt, mpm::G2PForm::kFast));
+    b->cur ^= 1;  // as mpm_g2p
+    b->substep += 1;
+    return MPM_OK;
 }
 
 static bool surrogate_cfg_ok(const MpmSurrogateConfig *c) {
@@ -524,7 +527,7 @@ int mpm_g2p_surrogate(MpmBuffers *b, const void *mlp_params, const MpmSurrogateC
     if (b->plan.n_particles > 0 && (!fallback || (reinterpret_cast<uintptr_t>(fallback) & 7))) return MPM_ERR_ARG;
     if (reinterpret_cast<uintptr_t>(mlp_params) & 15) return MPM_ERR_ARG;
     mpm::Ctx cx = make_ctx(b, stream, b->cur);
-    MPM_CHECK(mpm::launch_g2p(cx, dt, true));
+    MPM_CHECK(mpm::launch_g2p(cx, dt, mpm::G2PForm::kDeferStress));
     MPM_CHECK(mpm::launch_surrogate(cx, mlp_params, *cfg, static_cast<int2 *>(fallback), stats));
     b->cur ^= 1;  // as mpm_g2p: the updated records are in the other buffer
     b->substep += 1;

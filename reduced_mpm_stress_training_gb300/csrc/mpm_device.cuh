@@ -25,23 +25,23 @@ constexpr int kSvdSweeps = 5;           // Jacobi sweeps (converged in float32)
 // Views of the caller's buffers (layout fixed by mpm_plan).
 // ---------------------------------------------------------------------------
 // One particle-state buffer: a particle's 160-byte record (10 float4 quads)
-// split over three arrays -- quads 0-3 (64 B), 4-7 (64 B) and 8-9 (32 B) per
-// slot -- plus a cell-key array.  Record words (float unless noted):
-//   q0:  0-2 x_initial, 3 mass                                    array a
+// split over five arrays of quad pairs (32 B per slot) -- quads 0-1, 2-3, 4-5,
+// 6-7 and 8-9 -- plus a cell-key array.  Record words (float unless noted):
+//   q0:  0-2 x_initial, 3 mass                                    pair 0
 //   q1:  4 vol, 5 uid (int bits, the user's particle index), 6 yield_stress, 7 F[8]
-//   q2:  8-10 u, 11 v.x
+//   q2:  8-10 u, 11 v.x                                           pair 1
 //   q3:  12-13 v.y v.z, 14-15 C[0..1]
-//   q4:  16-19 C[2..5]                                            array b
+//   q4:  16-19 C[2..5]                                            pair 2
 //   q5:  20-22 C[6..8], 23 stress[0]
-//   q6:  24-27 stress[1..4]
+//   q6:  24-27 stress[1..4]                                       pair 3
 //   q7:  28-31 stress[5..8]
-//   q8:  32-35 F[0..3]                                            array f
+//   q8:  32-35 F[0..3]                                            pair 4
 //   q9:  36-39 F[4..7]
-// P2G reads q0-q7: one aligned 64-byte piece of a and one of b, so DRAM moves
-// exactly what it reads.  G2P reads q0, q1, q2 (one 64-byte piece of a) and
-// q8, q9 (32 B of f) and writes all three.  In one 160-byte array, each
-// kernel's partial reads dragged in nearly the whole record.  Matrices are
-// row-major as in the reference.
+// 32 bytes is both a DRAM sector and the widest load or store of one thread,
+// so a warp whose lanes hold consecutive slots moves a pair as 1 KB of
+// consecutive addresses with one instruction, straight from its registers
+// (no shared-memory staging), and a gather in user order still fetches whole
+// sectors.  Matrices are row-major as in the reference.
 constexpr int kRecWords = 40;
 constexpr int kRecQuads = 10;
 namespace rec {
@@ -49,20 +49,28 @@ constexpr int X0 = 0, MASS = 3, VOL = 4, UID = 5, YLD = 6, F8 = 7, U = 8, V = 11
               TAU = 23, F0 = 32;
 }
 struct PState {
-    float4 *a;    // quads 0-3 of each slot (padded stride)
-    float4 *b;    // quads 4-7
-    float4 *f;    // quads 8-9
+    float4 *q;    // pair p of slot s: q[(p * stride + s) * 2] and the quad after it
     int *key;     // cell key (block * 64 + cell in block) of each slot for the coming sort
     int64_t stride;
 };
 
 // address of record quad q (0..9) of a slot
 __device__ __forceinline__ float4 *recq(const PState &st, int slot, int q) {
-    return q < 4 ? st.a + (int64_t)slot * 4 + q
-                 : (q < 8 ? st.b + (int64_t)slot * 4 + (q - 4) : st.f + (int64_t)slot * 2 + (q - 8));
+    return st.q + ((int64_t)(q >> 1) * st.stride + slot) * 2 + (q & 1);
 }
 __device__ __forceinline__ float4 ldrec(const PState &st, int slot, int q) { return *recq(st, slot, q); }
 __device__ __forceinline__ void strec(const PState &st, int slot, int q, float4 v) { *recq(st, slot, q) = v; }
+// both quads of a pair in one 32-byte access (the state buffers are 256-byte aligned)
+__device__ __forceinline__ void ldpair(const PState &st, int slot, int p, float4 &a, float4 &b) {
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(recq(st, slot, 2 * p)));
+}
+__device__ __forceinline__ void stpair(const PState &st, int slot, int p, const float4 &a, const float4 &b) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(recq(st, slot, 2 * p)), "f"(a.x),
+                 "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
 // record word w (0..39) of a slot
 __device__ __forceinline__ float &recword(const PState &st, int slot, int w) {
     return reinterpret_cast<float *>(recq(st, slot, w >> 2))[w & 3];
@@ -192,6 +200,27 @@ __device__ __forceinline__ void warp_histogram(int *counts, int *cell_counts, in
     const int blk = key >= 0 ? (key >> 6) : -1;
     peers = __match_any_sync(0xffffffffu, blk);
     if (blk >= 0 && lane == __ffs(peers) - 1) atomicAdd(counts + blk, __popc(peers));
+}
+
+// The same counts for lanes whose particles came out of one cell-sorted chunk of
+// `block` (every lane of the warp calls it): most keep their cell, so equal
+// keys are neighbouring lanes and nearly all stay in the block.  One atomic per
+// run of equal keys, one for all the lanes still in the block, and one for
+// each that left it -- no match over the warp.
+__device__ __forceinline__ void sorted_histogram(int *counts, int *cell_counts, int key, int block) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int prev = __shfl_up_sync(full, key, 1);
+    const bool head = lane == 0 || prev != key;
+    const unsigned heads = __ballot_sync(full, head);
+    if (head && key >= 0) {
+        const unsigned later = lane < 31 ? heads >> (lane + 1) : 0u;
+        atomicAdd(cell_counts + key, later ? __ffs(later) : 32 - lane);
+    }
+    const int blk = key >= 0 ? (key >> 6) : -1;
+    const unsigned in = __ballot_sync(full, blk == block);
+    if (lane == 0 && in) atomicAdd(counts + block, __popc(in));
+    if (blk >= 0 && blk != block) atomicAdd(counts + blk, 1);
 }
 
 // ---------------------------------------------------------------------------

@@ -33,8 +33,11 @@ cudaError_t launch_p2g(const Ctx &cx, float dt);
 int64_t ordered_scratch_bytes(int64_t total_blocks);
 cudaError_t launch_p2g_ordered(const Ctx &cx, float dt, void *scratch);
 cudaError_t launch_grid(const Ctx &cx, float time, float dt);
-// defer_stress: store F_trial as F and skip the return map (surrogate stage follows)
-cudaError_t launch_g2p(const Ctx &cx, float dt, bool defer_stress = false);
+// kFast: the substep's form; kPinned: results that do not change from build to
+// build (the stage entry point and the ordered mode); kDeferStress: store
+// F_trial as F and skip the return map (surrogate stage follows)
+enum class G2PForm { kFast, kPinned, kDeferStress };
+cudaError_t launch_g2p(const Ctx &cx, float dt, G2PForm form);
 
 // surrogate stress stage (mpm_surrogate.cu): network stress with exact-invariant
 // correction and gating on the records G2P wrote into cx.st2; fallbacks to the

@@ -46,12 +46,6 @@ namespace mpm {
 // read-modify-writes of distinct nodes, no atomics).  At the block's end the
 // CTA sums the tiles that cover each node of the 6x6x6 tile and issues one
 // float4 atomicAdd per non-zero node.
-//
-// What it replaces: one warp per block with a whole stencil (108 accumulators)
-// per lane, which fit eight warps on an SM at a third of the issue rate.  Here
-// 24 warps fit and a block's latency is a quarter; the limit is shared-memory
-// bandwidth (the 25 numbers are read by nine lanes each).  Measured per launch:
-// 19.0 -> 8 us on 4,096 particles, 90 -> 79 us on the 1M column.
 // ---------------------------------------------------------------------------
 constexpr int kP2GWarps = 4;                  // one per x-slab of the block
 constexpr int kP2GQuads = 8;                  // record quads P2G reads (q0-q7, 128 B)
@@ -217,7 +211,7 @@ __global__ void __launch_bounds__(kP2GWarps * 32, 6) p2g_kernel(const MpmScene *
                 if (ok) {
                     float4 q[kP2GQuads];
 #pragma unroll
-                    for (int k = 0; k < kP2GQuads; ++k) q[k] = ldrec(st, slot, k);
+                    for (int k = 0; k < kP2GQuads; k += 2) ldpair(st, slot, k / 2, q[k], q[k + 1]);
                     ok = p2g_load(S, q, bx, by, bz, dt, o) && (__float_as_int(o[1].w) >> 4) == warp;
                 }
                 if (!ok) {  // contributes zeros
@@ -354,9 +348,13 @@ __global__ void __launch_bounds__(256) grid_kernel(const MpmScene *__restrict__ 
 // Software-pipelined over the CTA's chunks: while chunk k is computed, the
 // particle records (quads 0,1,2,8,9) and the 6x6x6 grid-velocity tile of
 // chunk k+1 stream into the other half of a double buffer in shared memory
-// with cp.async, and the order[] indices of chunk k+2 are loaded.  The
-// updated records are assembled in shared memory and written to their
-// (contiguous) sorted range with coalesced float4 stores.
+// with cp.async, and the order[] indices of chunk k+2 are loaded.  Each lane
+// writes its updated record straight to its sorted position, a quad pair per
+// 32-byte store (consecutive lanes, consecutive addresses).  Staging the
+// records in shared memory for stores of whole 64-byte pieces took 22 KB of
+// shared memory per CTA and 96 us per launch on the 1M column; this takes 86
+// us, and 80 us at five CTAs per SM.  It is bound by latency at 20 warps per
+// SM (57 % of the issue slots, 34 % of DRAM bandwidth).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int src_bytes) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -381,14 +379,22 @@ __device__ __forceinline__ V3 v3fma(float a, const V3 &x, const V3 &acc) {
 constexpr int kG2PQuads = 5;  // record quads G2P reads: 0, 1, 2, 8, 9
 __device__ __forceinline__ int g2p_quad(int q) { return q < 3 ? q : q + 5; }
 
-constexpr int kOutStride = kRecQuads + 1;  // padded so the per-thread record writes are conflict-free
-
 template <int CH>
 struct G2PSmem {
     float4 tile[2][kTileNodes];
     float4 rec[2][kG2PQuads][CH];
-    float4 outrec[CH * kOutStride];  // updated records of the chunk, written out coalesced
 };
+
+// a chunk's records (lanes of the chunk) into half b of the buffer
+template <int CH>
+__device__ __forceinline__ void g2p_prefetch_records(const PState &st, const Ws &ws, const int4 &ch, int slot,
+                                                     G2PSmem<CH> &sm, int b) {
+    if ((int)threadIdx.x < ch.z && ch.y + (int)threadIdx.x < ws.n) {
+#pragma unroll
+        for (int q = 0; q < kG2PQuads; ++q)
+            cp_async16(&sm.rec[b][q][threadIdx.x], recq(st, slot, g2p_quad(q)), 16);
+    }
+}
 
 // queue the async copies of one chunk into buffer b
 template <int CH>
@@ -396,11 +402,7 @@ __device__ __forceinline__ void g2p_prefetch(const MpmScene *__restrict__ scenes
                                              const Ws &ws, const int4 &ch, int slot,
                                              G2PSmem<CH> &sm, int b) {
     if (ch.w < 0) return;  // copy chunk: no compute, nothing to stage
-    if ((int)threadIdx.x < ch.z && ch.y + (int)threadIdx.x < ws.n) {
-#pragma unroll
-        for (int q = 0; q < kG2PQuads; ++q)
-            cp_async16(&sm.rec[b][q][threadIdx.x], recq(st, slot, g2p_quad(q)), 16);
-    }
+    g2p_prefetch_records<CH>(st, ws, ch, slot, sm, b);
     const MpmScene &S = scenes[ch.w];
     int bx, by, bz;
     chunk_block(S, ch.x, bx, by, bz);
@@ -414,6 +416,37 @@ __device__ __forceinline__ void g2p_prefetch(const MpmScene *__restrict__ scenes
     }
 }
 
+// The same copies with less integer work per chunk: the thread's tile nodes are
+// decoded once per CTA (x | y << 3 | z << 6 each), the node address comes from
+// the block id, and the chunk's block coordinates (x | y << 10 | z << 20; at most
+// 1024 blocks an axis) are handed to the chunk's compute.
+template <int CH>
+constexpr int kG2PTileIters = (kTileNodes + CH - 1) / CH;
+template <int CH>
+__device__ __forceinline__ void g2p_prefetch_fast(const MpmScene *__restrict__ scenes, const PState &st, const Ws &ws,
+                                                  const int4 &ch, int slot, const int (&tn)[kG2PTileIters<CH>],
+                                                  G2PSmem<CH> &sm, int b, int &blk) {
+    if (ch.w < 0) return;  // copy chunk: no compute, nothing to stage
+    g2p_prefetch_records<CH>(st, ws, ch, slot, sm, b);
+    const MpmScene &S = scenes[ch.w];
+    int bx, by, bz;
+    chunk_block(S, ch.x, bx, by, bz);
+    blk = bx | (by << 10) | (bz << 20);
+    const int nb = S.n_blocks_axis;
+    const int mx = S.n_grid - 4 * bx, my = S.n_grid - 4 * by, mz = S.n_grid - 4 * bz;
+#pragma unroll
+    for (int k = 0; k < kG2PTileIters<CH>; ++k) {
+        const int i = (int)threadIdx.x + k * CH;
+        if (i >= kTileNodes) break;
+        const int tx = tn[k] & 7, ty = (tn[k] >> 3) & 7, tz = tn[k] >> 6;
+        const bool in = tx < mx && ty < my && tz < mz;
+        const int gb = ch.x + ((tx >> 2) * nb + (ty >> 2)) * nb + (tz >> 2);
+        const int l = ((tx & 3) << 4) | ((ty & 3) << 2) | (tz & 3);
+        const float4 *src = ws.grid_v + (in ? (int64_t)gb * kBlockNodes + l : 0);
+        cp_async16(&sm.tile[b][i], src, in ? 16 : 0);  // outside the grid: zero fill
+    }
+}
+
 __device__ __forceinline__ int g2p_slot(const Ws &ws, const int4 &ch) {
     const int pos = ch.y + (int)threadIdx.x;
     return ((int)threadIdx.x < ch.z && pos < ws.n) ? ws.order[pos] : 0;
@@ -421,8 +454,13 @@ __device__ __forceinline__ int g2p_slot(const Ws &ws, const int4 &ch) {
 
 // DEFER: leave the return map and stress to a later pass (the surrogate stress
 // stage): F_trial is stored as F and the stress words are zeroed.
-template <int CH, bool DEFER>
-__global__ void __launch_bounds__(CH) g2p_kernel(const MpmScene *__restrict__ scenes, PState st,
+// FAST: the form that mpm_p2g2p runs, with five 128-thread CTAs per SM (96
+// registers) instead of four and less integer work.  The mpm_g2p stage and the
+// ordered mode run the other form: ptxas fuses multiplies and adds differently
+// under another register budget, and they promise float32 results that stay
+// the same bit for bit (see mpm_ordered.cu).
+template <int CH, bool DEFER, bool FAST>
+__global__ void __launch_bounds__(CH, FAST ? 640 / CH : 0) g2p_kernel(const MpmScene *__restrict__ scenes, PState st,
                                                  PState out, Ws ws, float dt, int *status) {
     extern __shared__ __align__(16) unsigned char g2p_smem_raw[];
     G2PSmem<CH> &sm = *reinterpret_cast<G2PSmem<CH> *>(g2p_smem_raw);
@@ -437,7 +475,18 @@ __global__ void __launch_bounds__(CH) g2p_kernel(const MpmScene *__restrict__ sc
     if (c >= n_chunks) return;
     int4 ch = ws.chunks[n_chunks - 1 - c];
     int slot = g2p_slot(ws, ch);
-    g2p_prefetch<CH>(scenes, st, ws, ch, slot, sm, 0);
+    [[maybe_unused]] int tn[kG2PTileIters<CH>];
+    [[maybe_unused]] int blk = 0, blkn = 0;
+    if constexpr (FAST) {
+#pragma unroll
+        for (int k = 0; k < kG2PTileIters<CH>; ++k) {
+            const int i = (int)threadIdx.x + k * CH;
+            tn[k] = i / 36 | ((i / 6) % 6) << 3 | (i % 6) << 6;
+        }
+        g2p_prefetch_fast<CH>(scenes, st, ws, ch, slot, tn, sm, 0, blk);
+    } else {
+        g2p_prefetch<CH>(scenes, st, ws, ch, slot, sm, 0);
+    }
     cp_async_commit();
     int cn = c + gridDim.x;
     int4 chn = make_int4(0, 0, 0, -1);
@@ -462,7 +511,11 @@ __global__ void __launch_bounds__(CH) g2p_kernel(const MpmScene *__restrict__ sc
         // barrier of the iteration
         cp_async_wait0();
         __syncthreads();
-        if (cn < n_chunks) g2p_prefetch<CH>(scenes, st, ws, chn, slotn, sm, buf ^ 1);
+        if constexpr (FAST) {
+            if (cn < n_chunks) g2p_prefetch_fast<CH>(scenes, st, ws, chn, slotn, tn, sm, buf ^ 1, blkn);
+        } else {
+            if (cn < n_chunks) g2p_prefetch<CH>(scenes, st, ws, chn, slotn, sm, buf ^ 1);
+        }
         cp_async_commit();
 
         const int pos = ch.y + (int)threadIdx.x;
@@ -478,7 +531,13 @@ __global__ void __launch_bounds__(CH) g2p_kernel(const MpmScene *__restrict__ sc
         } else if (mine) {
             const MpmScene &S = scenes[ch.w];
             int bx, by, bz;
-            chunk_block(S, ch.x, bx, by, bz);
+            if constexpr (FAST) {
+                bx = blk & 1023;
+                by = (blk >> 10) & 1023;
+                bz = blk >> 20;
+            } else {
+                chunk_block(S, ch.x, bx, by, bz);
+            }
             const float4 *tile = sm.tile[buf];
             const float4 q0 = sm.rec[buf][0][threadIdx.x], q1 = sm.rec[buf][1][threadIdx.x],
                          q2 = sm.rec[buf][2][threadIdx.x], q8 = sm.rec[buf][3][threadIdx.x],
@@ -496,12 +555,11 @@ __global__ void __launch_bounds__(CH) g2p_kernel(const MpmScene *__restrict__ sc
             }
             const int lx = base[0] - 4 * bx, ly = base[1] - 4 * by, lz = base[2] - 4 * bz;
             ok &= (unsigned)lx < 4u && (unsigned)ly < 4u && (unsigned)lz < 4u;
-            float4 *orec = sm.outrec + threadIdx.x * kOutStride;
             if (!ok) {
                 atomicOr(status, MPM_ST_INTERNAL);
                 key = sentinel;
 #pragma unroll
-                for (int q = 0; q < kRecQuads; ++q) orec[q] = ldrec(st, slot, q);
+                for (int q = 0; q < kRecQuads; ++q) strec(out, pos, q, ldrec(st, slot, q));
                 out.key[pos] = key;
             } else {
                 Weights W;
@@ -583,21 +641,20 @@ __global__ void __launch_bounds__(CH) g2p_kernel(const MpmScene *__restrict__ sc
                 } else {
                     return_map_stress(S, Ft, yld, Fo, tau);
                 }
-                // stores: record quads 1-9
+                // stores: the whole record at its sorted position
                 float chk = 0.0f;
 #pragma unroll
                 for (int k = 0; k < 9; ++k) chk += fabsf(Fo[k]) + fabsf(tau[k]);
                 if (!(S.material == MPM_METAL && S.hardening == 1)) yld = q1.z;
-                orec[0] = q0;
-                orec[1] = make_float4(q1.x, q1.y, yld, Fo[8]);
-                orec[2] = make_float4(un[0], un[1], un[2], nv[0]);
-                orec[3] = make_float4(nv[1], nv[2], nC[0], nC[1]);
-                orec[4] = make_float4(nC[2], nC[3], nC[4], nC[5]);
-                orec[5] = make_float4(nC[6], nC[7], nC[8], tau[0]);
-                orec[6] = make_float4(tau[1], tau[2], tau[3], tau[4]);
-                orec[7] = make_float4(tau[5], tau[6], tau[7], tau[8]);
-                orec[8] = make_float4(Fo[0], Fo[1], Fo[2], Fo[3]);
-                orec[9] = make_float4(Fo[4], Fo[5], Fo[6], Fo[7]);
+                stpair(out, pos, 0, q0, make_float4(q1.x, q1.y, yld, Fo[8]));
+                stpair(out, pos, 1, make_float4(un[0], un[1], un[2], nv[0]),
+                       make_float4(nv[1], nv[2], nC[0], nC[1]));
+                stpair(out, pos, 2, make_float4(nC[2], nC[3], nC[4], nC[5]),
+                       make_float4(nC[6], nC[7], nC[8], tau[0]));
+                stpair(out, pos, 3, make_float4(tau[1], tau[2], tau[3], tau[4]),
+                       make_float4(tau[5], tau[6], tau[7], tau[8]));
+                stpair(out, pos, 4, make_float4(Fo[0], Fo[1], Fo[2], Fo[3]),
+                       make_float4(Fo[4], Fo[5], Fo[6], Fo[7]));
                 int flags = 0;
                 const float vmax = S.dx / dt;
                 if (fabsf(nv[0]) > vmax || fabsf(nv[1]) > vmax || fabsf(nv[2]) > vmax) flags |= MPM_ST_CFL;
@@ -609,27 +666,12 @@ __global__ void __launch_bounds__(CH) g2p_kernel(const MpmScene *__restrict__ sc
                 out.key[pos] = key;
             }
         }
-        warp_histogram(ws.counts, ws.cell_counts, key);
-        // each warp writes out the records its own lanes staged
-        __syncwarp();
-        if (ch.w >= 0) {
-            // each warp writes its own 32 records, contiguous in each of the
-            // three arrays, with coalesced float4 stores: quads 0-3 to a and
-            // 4-7 to b (four per record), quads 8-9 to f (two per record)
-            const int w0 = (int)(threadIdx.x & ~31u);
-            const int np = max(0, min(min(32, ch.z - w0), ws.n - ch.y - w0));
-            const int64_t p0 = (int64_t)ch.y + w0;
-            const float4 *src = sm.outrec + w0 * kOutStride;
-            const int lane = (int)(threadIdx.x & 31u);
-            for (int l = lane; l < 4 * np; l += 32) {
-                const float4 *rq = src + (l >> 2) * kOutStride + (l & 3);
-                out.a[p0 * 4 + l] = rq[0];
-                out.b[p0 * 4 + l] = rq[4];
-            }
-            for (int l = lane; l < 2 * np; l += 32) out.f[p0 * 2 + l] = src[(l >> 1) * kOutStride + 8 + (l & 1)];
+        if constexpr (FAST) {
+            sorted_histogram(ws.counts, ws.cell_counts, key, ch.x);
+            blk = blkn;
+        } else {
+            warp_histogram(ws.counts, ws.cell_counts, key);
         }
-        // outrec and this half of the buffer are rewritten only after the next
-        // iteration's barrier, which every warp reaches after its write-out
         c = cn; ch = chn; slot = slotn;
         cn = cnn; chn = chnn; slotn = slotnn;
         buf ^= 1;
@@ -648,7 +690,7 @@ static int persistent_grid(const Ctx &cx, int per_sm) {
 // spread over the whole list instead of sweeping it as one band, and the L2
 // reuse with P2G (the chunk list walked from its end) would fall: 200.2 ->
 // 198.8 us per substep on the 1M column against twice the resident count.
-template <int CH, bool DEFER>
+template <int CH, bool DEFER, bool FAST>
 static cudaError_t g2p_t(const Ctx &cx, float dt) {
     // more than the 48 KB of static shared memory: opt in once per instance and device
     static int resident[64] = {0};
@@ -658,15 +700,15 @@ static cudaError_t g2p_t(const Ctx &cx, float dt) {
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (resident[dev] == 0) {
-        e = cudaFuncSetAttribute(g2p_kernel<CH, DEFER>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        e = cudaFuncSetAttribute(g2p_kernel<CH, DEFER, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return e;
         int nb = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, g2p_kernel<CH, DEFER>, CH, bytes);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, g2p_kernel<CH, DEFER, FAST>, CH, bytes);
         if (e != cudaSuccess) return e;
         resident[dev] = nb > 0 ? nb : 1;
     }
     const int grid = persistent_grid(cx, resident[dev]);
-    g2p_kernel<CH, DEFER><<<grid, CH, bytes, cx.stream>>>(cx.scenes, cx.st, cx.st2, cx.ws, dt, cx.status);
+    g2p_kernel<CH, DEFER, FAST><<<grid, CH, bytes, cx.stream>>>(cx.scenes, cx.st, cx.st2, cx.ws, dt, cx.status);
     return cudaGetLastError();
 }
 
@@ -698,19 +740,23 @@ cudaError_t launch_advance_colliders(MpmScene *scenes, int n_scenes, float time,
     return cudaGetLastError();
 }
 
-template <bool DEFER>
+template <bool DEFER, bool FAST>
 static cudaError_t g2p_sized(const Ctx &cx, float dt) {
     switch (cx.ws.chunk_size) {
-        case 32: return g2p_t<32, DEFER>(cx, dt);
-        case 64: return g2p_t<64, DEFER>(cx, dt);
-        case 128: return g2p_t<128, DEFER>(cx, dt);
-        case 256: return g2p_t<256, DEFER>(cx, dt);
+        case 32: return g2p_t<32, DEFER, FAST>(cx, dt);
+        case 64: return g2p_t<64, DEFER, FAST>(cx, dt);
+        case 128: return g2p_t<128, DEFER, FAST>(cx, dt);
+        case 256: return g2p_t<256, DEFER, FAST>(cx, dt);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t launch_g2p(const Ctx &cx, float dt, bool defer_stress) {
-    return defer_stress ? g2p_sized<true>(cx, dt) : g2p_sized<false>(cx, dt);
+cudaError_t launch_g2p(const Ctx &cx, float dt, G2PForm form) {
+    switch (form) {
+        case G2PForm::kFast: return g2p_sized<false, true>(cx, dt);
+        case G2PForm::kDeferStress: return g2p_sized<true, true>(cx, dt);
+        default: return g2p_sized<false, false>(cx, dt);
+    }
 }
 
 }  // namespace mpm

@@ -1,4 +1,4 @@
-"""P2G at the edges of its work split, against the float32 oracle: particle
+"""P2G and G2P at the edges of their work split.  P2G against the float32 oracle: particle
 counts around a warp's batch of 32 and its three groups, in one cell, in one
 x-slab of a grid block, in one block and over blocks that the grid cuts off;
 and blocks whose slabs are empty.
@@ -13,7 +13,7 @@ import torch
 
 from reduced_mpm_stress_training_gb300 import scenarios as S
 
-from helpers import gpu_sim, oracle_sim, rel
+from helpers import gpu_sim, gpu_state, oracle_sim, rel
 
 pytestmark = pytest.mark.gpu
 
@@ -60,3 +60,41 @@ def test_p2g_split_matches_oracle(cuda, where, n):
         assert rel(gvin.cpu().numpy(), ref.grid_v_in) < TOL
         e.stage("grid", time=0.0, dt=sc.dt)
     assert e.status() == 0
+
+
+@pytest.mark.parametrize("material", ["sand", "metal", "jelly"])
+@pytest.mark.parametrize("chunk", [32, 64, 128, 256])
+def test_substep_matches_its_stages(cuda, chunk, material):
+    """mpm_p2g2p's own G2P form against the mpm_g2p stage over three substeps, at
+    chunks that end inside a warp, blocks that the grid cuts off, particles that
+    change cell and block, and one outside the domain.  1e-5 relative, the
+    per-substep bar (the two round differently)."""
+    rng = np.random.default_rng(chunk)
+    n = 2 * chunk + 37
+    kw = dict(E=2e5, density=2000.0, yield_stress=2e3, hardening=1, xi=0.1) if material == "metal" else {}
+    sc = S.small_column(n, N_GRID, material="metal" if material == "metal" else "sand", **kw)
+    sc.material = material
+    x0 = (rng.uniform(4.0, 15.4, (n, 3)) / N_GRID).astype(np.float32)
+    x0[: chunk + 5] = (rng.uniform(13.6, 15.4, (chunk + 5, 3)) / N_GRID).astype(np.float32)  # one edge block
+    x0[-1] = 1.5
+    v = (40.0 * rng.normal(size=(n, 3))).astype(np.float32)  # up to about half a cell a substep
+    F = (np.eye(3) + 0.02 * rng.normal(size=(n, 3, 3)) - 0.03 * np.eye(3)).astype(np.float32)
+    vol = np.full(n, 1e-5, np.float32)
+    mass = np.full(n, 2e-2, np.float32)
+    out = []
+    for whole in (True, False):
+        sim = gpu_sim(sc, chunk_size=chunk, x0=x0, v0=v, vol=vol, mass=mass)
+        sim.on_error = "ignore"
+        sim.load_F_from_tensor(torch.from_numpy(F))
+        e = sim.engine
+        for _ in range(3):
+            if whole:
+                e.substep_raw(0.0, sc.dt)
+            else:
+                for name in ("sort", "p2g", "grid", "g2p"):
+                    e.stage(name, time=0.0, dt=sc.dt)
+        out.append(gpu_state(sim))
+        e.clear_status()
+    for f in ("x", "v", "F", "yield_"):
+        assert rel(out[0][f], out[1][f]) < TOL, f
+    assert np.isfinite(out[0]["stress"]).all()
