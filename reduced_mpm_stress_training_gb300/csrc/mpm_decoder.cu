@@ -207,6 +207,14 @@ __global__ void __launch_bounds__(kDecThreads) decoder_rows_kernel(MpmStressDeco
     }
 }
 
+// the symmetric stress of the six components into the record, whole pairs (sectors) at a time
+__device__ __forceinline__ void store_stress(const PState &st, int i, const float q[6]) {
+    float4 q4, q5;
+    ldpair(st, i, 2, q4, q5);
+    stpair(st, i, 2, q4, make_float4(q5.x, q5.y, q5.z, q[0]));
+    stpair(st, i, 3, make_float4(q[1], q[2], q[1], q[3]), make_float4(q[4], q[2], q[4], q[5]));
+}
+
 // The decoder as the stress source of a substep: label (label_dim floats, the
 // frame's latent), each particle's x_initial from its record and mu row
 // (mu_dim floats, user order) by uid; writes the symmetric stress
@@ -250,10 +258,7 @@ __global__ void __launch_bounds__(kDecThreads) decoder_stress_kernel(MpmStressDe
         for (int j = 0; j < HP; ++j) h[j] = dec_act(h[j], siren, d.omega_0);
         float q[6];
         dec_tail<HP>(sm, L, h, siren, d.omega_0, q);
-        const float4 q5 = ldrec(st, i, 5);
-        strec(st, i, 5, make_float4(q5.x, q5.y, q5.z, q[0]));
-        strec(st, i, 6, make_float4(q[1], q[2], q[1], q[3]));
-        strec(st, i, 7, make_float4(q[4], q[2], q[4], q[5]));
+        store_stress(st, i, q);
     }
 }
 
@@ -519,10 +524,7 @@ __global__ void __launch_bounds__(P * dtc::kRows, P == 2 ? 3 : 4) decoder_stress
             q[c] = __fadd_rn(s.qm[c], __fmul_rn(acc, s.qs[c]));
         }
         if (live) {
-            const float4 q5 = ldrec(st, i, 5);
-            strec(st, i, 5, make_float4(q5.x, q5.y, q5.z, q[0]));
-            strec(st, i, 6, make_float4(q[1], q[2], q[1], q[3]));
-            strec(st, i, 7, make_float4(q[4], q[2], q[4], q[5]));
+            store_stress(st, i, q);
         }
     }
     if (!ok && row == 0) {
