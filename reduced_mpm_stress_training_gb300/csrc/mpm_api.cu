@@ -50,10 +50,10 @@ inline int64_t align_up(int64_t x, int64_t a = kAlign) { return (x + a - 1) / a 
 constexpr int64_t kStateBytesPerParticle = mpm::kRecWords * 4 + 4;
 
 struct WsLayout {
-    int64_t order, counts, cell_counts, cell_start, cell_cursor, tile_sums, ticket, chunks, n_chunks,
+    int64_t order, counts, cell_counts, cell_start, cell_cursor, tile_sums, chunks, n_chunks,
         blocks, n_blocks, grid_acc, grid_v, block_flag, active_list, n_active, n_active_prev, staging,
         slot_of_uid, total;
-    int nbk, n_tiles;
+    int nbk;
 };
 
 WsLayout ws_layout(const MpmPlan &p) {
@@ -61,7 +61,6 @@ WsLayout ws_layout(const MpmPlan &p) {
     const int64_t n = p.particle_stride;
     const int64_t nbk = p.total_blocks + 1;
     L.nbk = (int)nbk;
-    L.n_tiles = (int)((nbk + mpm::kScanTile - 1) / mpm::kScanTile);
     int64_t o = 0;
     auto take = [&](int64_t bytes) { int64_t at = o; o = align_up(o + bytes); return at; };
     L.order = take(n * 4);
@@ -69,8 +68,8 @@ WsLayout ws_layout(const MpmPlan &p) {
     L.cell_counts = take(nbk * 64 * 4);
     L.cell_start = take(nbk * 64 * 4);
     L.cell_cursor = take(nbk * 64 * 4);
-    L.tile_sums = take((int64_t)L.n_tiles * 16);
-    L.ticket = take(4);
+    L.tile_sums = take((nbk + 511) / 512 * 16);
+    take(4);  // (a slot that keeps the later offsets and the total as they were)
     L.chunks = take(p.max_chunks * 16);
     L.n_chunks = take(4);
     L.blocks = take((p.total_blocks + 1) * 16);
@@ -128,7 +127,6 @@ mpm::Ctx make_ctx(const MpmBuffers *b, void *stream, int which) {
     ws.cell_start = reinterpret_cast<int *>(w + L.cell_start);
     ws.cell_cursor = reinterpret_cast<int *>(w + L.cell_cursor);
     ws.tile_sums = reinterpret_cast<int4 *>(w + L.tile_sums);
-    ws.ticket = reinterpret_cast<unsigned *>(w + L.ticket);
     ws.chunks = reinterpret_cast<int4 *>(w + L.chunks);
     ws.n_chunks = reinterpret_cast<int *>(w + L.n_chunks);
     ws.blocks = reinterpret_cast<int4 *>(w + L.blocks);
@@ -142,7 +140,6 @@ mpm::Ctx make_ctx(const MpmBuffers *b, void *stream, int which) {
     ws.staging = reinterpret_cast<float *>(w + L.staging);
     ws.slot_of_uid = reinterpret_cast<int *>(w + L.slot_of_uid);
     ws.nbk = L.nbk;
-    ws.n_tiles = L.n_tiles;
     ws.max_chunks = (int)p.max_chunks;
     ws.chunk_size = p.chunk_size;
     ws.n = (int)p.n_particles;

@@ -13,12 +13,7 @@ namespace mpm {
 constexpr int kTile = 6;                // padded node tile per 4^3-cell block
 constexpr int kTileNodes = kTile * kTile * kTile;  // 216
 constexpr int kBlockNodes = 64;         // nodes of one 4x4x4 grid block
-// one bucket per thread, 16 warps per scan tile: scan_finish's per-block cell
-// scans spread over twice the warps of a 256-thread CTA with two buckets each
-// (measured 34.9 -> 30.9 us per sort on the 1M column)
-constexpr int kScanThreads = 512;      // threads per scan CTA
-constexpr int kScanPerThread = 1;      // buckets per scan thread
-constexpr int kScanTile = kScanThreads * kScanPerThread;  // buckets per scan CTA
+constexpr int kScanThreads = 256;      // threads per scan CTA
 constexpr int kSvdSweeps = 5;           // Jacobi sweeps (converged in float32)
 
 // ---------------------------------------------------------------------------
@@ -82,8 +77,7 @@ struct Ws {  // workspace
     int *cell_counts;  // particles per cell (64 per block)
     int *cell_start;   // first sorted position of each cell
     int *cell_cursor;  // scatter cursor of each cell; equals the cell end afterwards
-    int4 *tile_sums;  // per scan tile: (particles, chunks, non-empty blocks)
-    unsigned *ticket;
+    int4 *tile_sums;  // per 512 buckets: (particles, chunks, non-empty blocks)
     int4 *chunks;     // G2P work: (global block, start, count <= chunk_size, scene)
     int *n_chunks;
     int4 *blocks;     // P2G work: (global block, start, count, scene), one per non-empty block
@@ -97,7 +91,6 @@ struct Ws {  // workspace
     float *staging;
     int *slot_of_uid;  // user particle -> slot of the live state (host transfers)
     int nbk;          // buckets = total_blocks + 1 (last = out of domain)
-    int n_tiles;
     int max_chunks;
     int chunk_size;
     int n;            // particles (bounds every order[] index)

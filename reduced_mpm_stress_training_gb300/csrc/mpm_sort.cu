@@ -10,10 +10,9 @@
 //   keys + histograms -- written by G2P for the next substep (block and
 //                        cell counts), or by key_kernel after a load moved
 //                        particles
-//   scan_tiles        -- per-tile sums of the block counts; the last CTA to
-//                        finish scans the tile sums (atomic ticket, no spin)
-//   scan_finish       -- block offsets, the P2G block list and the G2P chunk
+//   scan              -- block offsets, the P2G block list and the G2P chunk
 //                        list; for each non-empty block, its 64 cell offsets
+//                        (after bucket_sums on large grids)
 //   scatter           -- order[] via warp-aggregated cell-cursor atomics
 // G2P then writes every record to the other state buffer at its sorted
 // position, so order[] stays close to the identity from one substep to the
@@ -44,8 +43,8 @@ __device__ __forceinline__ int4 add4(int4 a, int4 b) {
     return make_int4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
 
-// inclusive scan of an int4 triple over the kScanThreads threads of a CTA;
-// returns the thread's inclusive value and leaves the CTA total in *total
+// inclusive scan of an int4 over the kScanThreads threads of a CTA; returns
+// the thread's inclusive value and leaves the CTA total in total
 constexpr int kScanWarps = kScanThreads / 32;
 __device__ __forceinline__ int4 cta_scan4(int4 v, int4 *wsum /* [kScanWarps] shared */, int4 &total) {
     int4 x = v;
@@ -55,7 +54,7 @@ __device__ __forceinline__ int4 cta_scan4(int4 v, int4 *wsum /* [kScanWarps] sha
         y.x = __shfl_up_sync(0xffffffffu, x.x, o);
         y.y = __shfl_up_sync(0xffffffffu, x.y, o);
         y.z = __shfl_up_sync(0xffffffffu, x.z, o);
-        y.w = 0;
+        y.w = __shfl_up_sync(0xffffffffu, x.w, o);
         if ((threadIdx.x & 31) >= o) x = add4(x, y);
     }
     if ((threadIdx.x & 31) == 31) wsum[threadIdx.x >> 5] = x;
@@ -78,106 +77,111 @@ __device__ __forceinline__ int4 bucket_triple(const Ws &ws, int b, int cnt) {
     return make_int4(cnt, ch, cnt > 0 ? 1 : 0, 0);
 }
 
-// Phase 1: per-tile sums.  The last CTA to finish (atomic ticket; nobody
-// waits) scans the tile sums into exclusive tile offsets and publishes the
-// work-list lengths.
-__global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(Ws ws) {
-    __shared__ int4 wsum[kScanWarps];
-    __shared__ bool last;
-    const int tile = blockIdx.x;
-    const int b0 = tile * kScanTile + threadIdx.x * kScanPerThread;
-    int4 acc = make_int4(0, 0, 0, 0);
-#pragma unroll
-    for (int j = 0; j < kScanPerThread; ++j) {
-        int b = b0 + j;
-        if (b < ws.nbk) acc = add4(acc, bucket_triple(ws, b, ws.counts[b]));
-    }
-    int4 total;
-    cta_scan4(acc, wsum, total);
-    if (threadIdx.x == 0) {
-        ws.tile_sums[tile] = total;
-        __threadfence();
-        unsigned t = atomicAdd(ws.ticket, 1u);
-        last = (t == (unsigned)gridDim.x - 1);
-    }
+// sum of an int4 over the kScanThreads threads of a CTA (every thread gets it)
+__device__ __forceinline__ int4 cta_sum4(int4 v, int4 *wsum /* [kScanWarps] shared */) {
+    v.x = __reduce_add_sync(0xffffffffu, v.x);
+    v.y = __reduce_add_sync(0xffffffffu, v.y);
+    v.z = __reduce_add_sync(0xffffffffu, v.z);
+    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = v;
     __syncthreads();
-    if (!last) return;
-    __threadfence();
-    int4 carry = make_int4(0, 0, 0, 0);
-    for (int base = 0; base < ws.n_tiles; base += kScanThreads) {
-        const int t = base + threadIdx.x;
-        int4 v = t < ws.n_tiles ? __ldcg(ws.tile_sums + t) : make_int4(0, 0, 0, 0);
-        int4 tot;
-        int4 inc = cta_scan4(v, wsum, tot);
-        if (t < ws.n_tiles) {
-            int4 ex = add4(carry, make_int4(inc.x - v.x, inc.y - v.y, inc.z - v.z, 0));
-            ws.tile_sums[t] = ex;
-        }
-        carry = add4(carry, tot);
-    }
-    if (threadIdx.x == 0) {
-        // counts always sum to n when the stages run in order; the clamps keep
-        // a mis-sequenced call from walking past the work lists
-        *ws.n_chunks = min(carry.y, ws.max_chunks);
-        *ws.n_blocks = min(carry.z, ws.nbk - 1);
-        *ws.ticket = 0u;  // re-arm for the next substep
-    }
+    int4 t = make_int4(0, 0, 0, 0);
+    for (int w = 0; w < kScanWarps; ++w) t = add4(t, wsum[w]);
+    __syncthreads();
+    return t;
 }
 
-// Phase 2: bucket offsets / cursors, the G2P chunk list and the P2G block
-// list; zeroes the histogram for the next substep.  Each thread first finds
-// the offsets of its buckets (a CTA scan on top of the tile's exclusive
-// prefix); then the CTA's warps take its non-empty buckets one at a time and
-// write the 64 cell offsets of each with a warp scan (two cells per lane),
-// and its chunk-list entries with one lane per chunk.
-__global__ void __launch_bounds__(kScanThreads) scan_finish_kernel(const MpmScene *__restrict__ scenes,
-                                                          int n_scenes, Ws ws) {
+// Sums of kSumTile buckets each, for grids too large for scan_kernel to add up
+// the counts themselves.
+constexpr int kSumTile = 512;
+__global__ void __launch_bounds__(kScanThreads) bucket_sums_kernel(Ws ws) {
     __shared__ int4 wsum[kScanWarps];
-    __shared__ int s_off[kScanTile], s_coff[kScanTile], s_boff[kScanTile], s_cnt[kScanTile];
-    __shared__ int s_list[kScanTile];
-    __shared__ int s_nlist;
-    const int tile = blockIdx.x;
-    const int b0 = tile * kScanTile + threadIdx.x * kScanPerThread;
-    if (threadIdx.x == 0) s_nlist = 0;
-    const int4 pre = ws.tile_sums[tile];  // loaded beside the counts: one round trip for both
-    int cnt[kScanPerThread];
     int4 acc = make_int4(0, 0, 0, 0);
 #pragma unroll
-    for (int j = 0; j < kScanPerThread; ++j) {
-        int b = b0 + j;
-        cnt[j] = b < ws.nbk ? ws.counts[b] : 0;
-        if (b < ws.nbk) acc = add4(acc, bucket_triple(ws, b, cnt[j]));
+    for (int k = 0; k < kSumTile / kScanThreads; ++k) {
+        const int b = blockIdx.x * kSumTile + k * kScanThreads + (int)threadIdx.x;
+        if (b < ws.nbk) acc = add4(acc, bucket_triple(ws, b, ws.counts[b]));
     }
+    const int4 t = cta_sum4(acc, wsum);
+    if (threadIdx.x == 0) ws.tile_sums[blockIdx.x] = t;
+}
+
+// Bucket offsets / cursors, the G2P chunk list and the P2G block list.  A CTA
+// owns KB buckets and finds what lies before them by itself, so no
+// CTA waits for another and no pass over tile sums comes in between: from the
+// counts of all earlier buckets (SUMS false: a few independent loads a thread
+// while there are at most kDirectBuckets of them), or from bucket_sums_kernel's
+// sums.  Then its warps take its non-empty buckets and write the 64 cell
+// offsets of each with a warp scan (two cells per lane), and its chunk-list
+// entries with one lane per chunk.  The last CTA publishes the list lengths.
+// (A kernel that scanned all tile sums behind an atomic ticket cost 5 to 12 us a
+// substep.  Handing the ranges out with atomics, in the order CTAs arrive, is as
+// fast here but scatters neighbouring blocks: P2G 3 % slower on 64 scenes.)
+constexpr int kDirectBuckets = 8192;  // an 80^3 grid: up to eight 16-byte loads a thread
+// KB buckets per CTA: the non-empty blocks of a column lie side by side, so a
+// few CTAs hold most of them and need the warps (64 buckets a CTA instead of
+// 256: sort of the 1M column 26.8 -> 22.5 us).  Past kWideBuckets there are
+// CTAs enough, and each one's sum over the tile sums counts (256 instead of 64:
+// 64 scenes, 420k buckets, 74 -> 62 us).
+constexpr int kWideBuckets = 1 << 17;
+template <bool SUMS, int KB>
+__global__ void __launch_bounds__(kScanThreads) scan_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
+                                                            Ws ws) {
+    __shared__ int4 wsum[kScanWarps];
+    __shared__ int s_off[KB], s_coff[KB], s_boff[KB], s_cnt[KB];
+    __shared__ int s_list[KB];
+    const int tile = blockIdx.x;
+    const int b0 = tile * KB;
+    const bool owner = (int)threadIdx.x < KB;  // of bucket b
+    const int b = owner ? b0 + (int)threadIdx.x : ws.nbk;
+    const int cnt = b < ws.nbk ? ws.counts[b] : 0;
+    // what lies before the CTA's buckets (b0 is a multiple of four, and no bucket
+    // before it is the sentinel, the last one)
+    int4 pre = make_int4(0, 0, 0, 0);
+    if (SUMS) {
+        const int full = b0 / kSumTile;
+        for (int t = threadIdx.x; t < full; t += kScanThreads) pre = add4(pre, ws.tile_sums[t]);
+        for (int h = full * kSumTile + (int)threadIdx.x; h < b0; h += kScanThreads)
+            pre = add4(pre, bucket_triple(ws, h, ws.counts[h]));
+    } else {
+        const int4 *c4 = reinterpret_cast<const int4 *>(ws.counts);
+#pragma unroll 8
+        for (int i = threadIdx.x; i < b0 / 4; i += kScanThreads) {
+            const int4 c = c4[i];
+            pre = add4(pre, add4(add4(bucket_triple(ws, 0, c.x), bucket_triple(ws, 0, c.y)),
+                                 add4(bucket_triple(ws, 0, c.z), bucket_triple(ws, 0, c.w))));
+        }
+    }
+    pre = cta_sum4(pre, wsum);
+    int4 mine = b < ws.nbk ? bucket_triple(ws, b, cnt) : make_int4(0, 0, 0, 0);
+    // the out-of-domain bucket always gets its cursor (G2P's copy chunks count its particles again)
+    const bool listed = b < ws.nbk && (cnt > 0 || b == ws.nbk - 1);
+    mine.w = listed ? 1 : 0;
     int4 total;
-    int4 inc = cta_scan4(acc, wsum, total);  // its barriers also order s_nlist = 0
-    int off = pre.x + inc.x - acc.x, coff = pre.y + inc.y - acc.y, boff = pre.z + inc.z - acc.z;
-#pragma unroll
-    for (int j = 0; j < kScanPerThread; ++j) {
-        const int b = b0 + j;
-        if (b >= ws.nbk) break;
-        ws.counts[b] = 0;
-        const int li = threadIdx.x * kScanPerThread + j;
-        s_off[li] = off;
-        s_coff[li] = coff;
-        s_boff[li] = boff;
-        s_cnt[li] = cnt[j];
-        // the out-of-domain bucket always gets its cursor (its particles sort
-        // after every other one; G2P's copy chunks count them again)
-        if (cnt[j] > 0 || b == ws.nbk - 1) s_list[atomicAdd(&s_nlist, 1)] = li;
-        const int4 t = bucket_triple(ws, b, cnt[j]);
-        off += t.x;
-        coff += t.y;
-        boff += t.z;
+    const int4 inc = cta_scan4(mine, wsum, total);
+    const int nlist = total.w;
+    if (listed) s_list[inc.w - 1] = (int)threadIdx.x;
+    if (owner) {
+        s_off[threadIdx.x] = pre.x + inc.x - mine.x;
+        s_coff[threadIdx.x] = pre.y + inc.y - mine.y;
+        s_boff[threadIdx.x] = pre.z + inc.z - mine.z;
+        s_cnt[threadIdx.x] = cnt;
     }
-    __syncthreads();
+    if (threadIdx.x == 0 && tile == (int)gridDim.x - 1) {
+        // counts always sum to n when the stages run in order; the clamps keep
+        // a mis-sequenced call from walking past the work lists
+        *ws.n_chunks = min(pre.y + total.y, ws.max_chunks);
+        *ws.n_blocks = min(pre.z + total.z, ws.nbk - 1);
+        *ws.n_active_prev = *ws.n_active;
+        *ws.n_active = 0;
+    }
     const int lane = threadIdx.x & 31;
-    const int nlist = s_nlist;
     const int cs = ws.chunk_size;
     // a warp takes kScanPrefetch of the tile's non-empty buckets at a time and
     // loads all their cell counts before scanning any, so the loads' round
     // trips overlap instead of queueing one after another
     constexpr int kScanPrefetch = 8;
     const int warp = (int)(threadIdx.x >> 5);
+    __syncthreads();
     for (int i0 = warp; i0 < nlist; i0 += kScanWarps * kScanPrefetch) {
         int lis[kScanPrefetch];
         int2 ks[kScanPrefetch];
@@ -185,15 +189,15 @@ __global__ void __launch_bounds__(kScanThreads) scan_finish_kernel(const MpmScen
         for (int u = 0; u < kScanPrefetch; ++u) {
             const int i = i0 + u * kScanWarps;
             lis[u] = i < nlist ? s_list[i] : -1;
-            ks[u] = lis[u] >= 0
-                        ? reinterpret_cast<const int2 *>(ws.cell_counts + (int64_t)(tile * kScanTile + lis[u]) * 64)[lane]
-                        : make_int2(0, 0);
+            ks[u] = lis[u] >= 0 ? reinterpret_cast<const int2 *>(
+                                      ws.cell_counts + (int64_t)(b0 + lis[u]) * 64)[lane]
+                                : make_int2(0, 0);
         }
 #pragma unroll
         for (int u = 0; u < kScanPrefetch; ++u) {
             const int li = lis[u];
             if (li < 0) break;  // uniform over the warp
-            const int b = tile * kScanTile + li;
+            const int bk = b0 + li;
             const int bo = s_off[li], n_b = s_cnt[li];
             // cell offsets of the block: lane owns cells 2 lane, 2 lane + 1
             const int2 k = ks[u];
@@ -206,24 +210,21 @@ __global__ void __launch_bounds__(kScanThreads) scan_finish_kernel(const MpmScen
             }
             const int st = bo + incl - sum;
             const int2 st2 = make_int2(st, st + k.x);
-            reinterpret_cast<int2 *>(ws.cell_start + (int64_t)b * 64)[lane] = st2;
-            reinterpret_cast<int2 *>(ws.cell_cursor + (int64_t)b * 64)[lane] = st2;
-            reinterpret_cast<int2 *>(ws.cell_counts + (int64_t)b * 64)[lane] = make_int2(0, 0);
+            reinterpret_cast<int2 *>(ws.cell_start + (int64_t)bk * 64)[lane] = st2;
+            reinterpret_cast<int2 *>(ws.cell_cursor + (int64_t)bk * 64)[lane] = st2;
+            reinterpret_cast<int2 *>(ws.cell_counts + (int64_t)bk * 64)[lane] = make_int2(0, 0);
             if (n_b > 0) {
-                const bool real = b < ws.nbk - 1;
-                const int sc = real ? scene_of_block(scenes, n_scenes, b) : -1;  // -1: copy chunk
-                if (real && lane == 0 && s_boff[li] < ws.nbk - 1) ws.blocks[s_boff[li]] = make_int4(b, bo, n_b, sc);
+                const bool real = bk < ws.nbk - 1;
+                const int sc = real ? scene_of_block(scenes, n_scenes, bk) : -1;  // -1: copy chunk
+                const int at_b = s_boff[li];
+                if (real && lane == 0 && at_b < ws.nbk - 1) ws.blocks[at_b] = make_int4(bk, bo, n_b, sc);
                 const int nch = (n_b + cs - 1) / cs;
                 for (int c = lane; c < nch; c += 32) {
                     const int at = s_coff[li] + c;
-                    if (at < ws.max_chunks) ws.chunks[at] = make_int4(b, bo + c * cs, min(cs, n_b - c * cs), sc);
+                    if (at < ws.max_chunks) ws.chunks[at] = make_int4(bk, bo + c * cs, min(cs, n_b - c * cs), sc);
                 }
             }
         }
-    }
-    if (tile == 0 && threadIdx.x == 0) {
-        *ws.n_active_prev = *ws.n_active;
-        *ws.n_active = 0;
     }
 }
 
@@ -231,7 +232,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_finish_kernel(const MpmScen
 // kScatterPer keys (strided by the grid's thread count) so that their
 // cursor atomics are in flight together.  Also zeroes the grid accumulator
 // of the previous substep's active blocks (kept until now so grid mass and
-// momentum stay readable between substeps).
+// momentum stay readable between substeps) and the block counts that the scan
+// has read, for G2P to count into.
 constexpr int kScatterPer = 4;
 
 __global__ void __launch_bounds__(256) scatter_kernel(PState st, Ws ws, int n) {
@@ -246,6 +248,7 @@ __global__ void __launch_bounds__(256) scatter_kernel(PState st, Ws ws, int n) {
         const int64_t idx = (int64_t)i + (int64_t)r * stride;
         key[r] = idx < n ? __ldcs(st.key + idx) : -1;
     }
+    for (int j = i; j < ws.nbk; j += stride) ws.counts[j] = 0;
     const int nclear = *ws.n_active_prev * kBlockNodes;
     for (int j = i; j < nclear; j += stride)
         ws.grid_acc[(int64_t)ws.active_list[j >> 6] * kBlockNodes + (j & 63)] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -274,8 +277,16 @@ cudaError_t launch_keys(const Ctx &cx) {
 }
 
 cudaError_t launch_sort(const Ctx &cx) {
-    scan_tiles_kernel<<<cx.ws.n_tiles, kScanThreads, 0, cx.stream>>>(cx.ws);
-    scan_finish_kernel<<<cx.ws.n_tiles, kScanThreads, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.ws);
+    const int nbk = cx.ws.nbk;
+    if (nbk <= kDirectBuckets) {
+        scan_kernel<false, 64><<<(nbk + 63) / 64, kScanThreads, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.ws);
+    } else {
+        bucket_sums_kernel<<<(nbk + kSumTile - 1) / kSumTile, kScanThreads, 0, cx.stream>>>(cx.ws);
+        if (nbk <= kWideBuckets)
+            scan_kernel<true, 64><<<(nbk + 63) / 64, kScanThreads, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.ws);
+        else
+            scan_kernel<true, 256><<<(nbk + 255) / 256, kScanThreads, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.ws);
+    }
     const int per = 256 * kScatterPer;
     const int sgrid = cx.n > 0 ? (cx.n + per - 1) / per : 1;
     scatter_kernel<<<sgrid, 256, 0, cx.stream>>>(cx.st, cx.ws, cx.n);

@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 import torch
 
+from reduced_mpm_stress_training_gb300 import _capi as A
 from reduced_mpm_stress_training_gb300 import scenarios as S
 
 from helpers import gpu_sim, gpu_state, oracle_sim, rel
@@ -98,3 +99,38 @@ def test_substep_matches_its_stages(cuda, chunk, material):
     for f in ("x", "v", "F", "yield_"):
         assert rel(out[0][f], out[1][f]) < TOL, f
     assert np.isfinite(out[0]["stress"]).all()
+
+
+@pytest.mark.parametrize("n_grid", [4, 15, 16, 80, 84, 200, 204])
+def test_sort_over_grid_sizes(cuda, n_grid):
+    """The sort's scan at its changes of form (8,192 and 131,072 buckets) and at
+    grids of one to a few CTAs: particles over the whole grid, first and last
+    blocks included, some outside; two substeps, the second on G2P's counts.
+    Grid mass against the oracle, and every particle in some cell."""
+    rng = np.random.default_rng(n_grid)
+    n = 3000
+    sc = S.small_column(n, n_grid, gravity=(0.0, 0.0, 0.0))
+    x0 = ((0.5 + rng.uniform(0.01, n_grid - 2.01, (n, 3))) / n_grid).astype(np.float32)
+    x0[0] = 0.51 / n_grid
+    x0[1] = (n_grid - 1.51) / n_grid
+    x0[7::100] += 2.0  # outside the domain
+    inside = (x0 < 1.5).all(1)
+    vol = np.full(n, 1e-6, np.float32)
+    mass = rng.uniform(1.0, 2.0, n).astype(np.float32)
+    v = np.zeros((n, 3), np.float32)
+    sim = gpu_sim(sc, x0=x0, v0=v, vol=vol, mass=mass, colliders=False)
+    sim.on_error = "ignore"
+    k = int(inside.sum())
+    ref = oracle_sim(S.small_column(k, n_grid, gravity=(0.0, 0.0, 0.0)), x0=x0[inside], v0=v[inside], vol=vol[inside],
+                     mass=mass[inside], colliders=False)
+    ref.stage_p2g(sc.dt)
+    e = sim.engine
+    for _ in range(2):  # at rest and without gravity nothing moves
+        e.stage("sort")
+        e.stage("p2g", dt=sc.dt)
+        gm, _, _ = e.export_grid(0)
+        assert rel(gm.cpu().numpy(), ref.grid_m) < TOL
+        e.stage("grid", time=0.0, dt=sc.dt)
+        e.stage("g2p", dt=sc.dt)
+    assert torch.equal(e.export(A.FIELD_MASS).cpu(), torch.from_numpy(mass))
+    e.clear_status()
