@@ -113,26 +113,68 @@ __global__ void __launch_bounds__(256) mark_kernel(const MpmScene *__restrict__ 
     }
 }
 
-// p2g_sample_all (mpm_utils.py:353-402): one thread per particle record.  A
-// particle whose base cell is marked sets F = F_disp + I, takes the stress of
-// that F (FCR for jelly and metal, Drucker-Prager for sand; :368-378) and
-// scatters, per node, w m v + dt (-(m / density) stress grad w) and w m.
-// The records are sorted by cell, so neighbouring lanes mostly share a base
-// cell and hit the same 27 nodes: each node's contributions are summed over
-// every run of lanes with one base cell (a segmented shuffle reduction) and
-// the run's first lane issues one 16-byte atomic for it.
-__global__ void __launch_bounds__(256) reduced_p2g_kernel(const MpmScene *__restrict__ scenes, PState st,
-                                                          MpmReducedGrid g, int n, float dt, int *status) {
+// The Drucker-Prager Kirchhoff stress of F without an SVD: tau = 2 mu E +
+// lam tr(E) I with E = log(F F^T) / 2, in Newton form on the closed-form
+// eigenvalues of B = F F^T - I (as sand_return_map_spectral, which also says
+// why it is the more accurate form near F = I).  False (SVD path) for inverted
+// or extremely compressed elements.
+__device__ __forceinline__ bool stress_dp_spectral(const float F[9], float mu, float lam, float tau[9]) {
+    const float J = F[0] * (F[4] * F[8] - F[5] * F[7]) - F[1] * (F[3] * F[8] - F[5] * F[6]) +
+                    F[2] * (F[3] * F[7] - F[4] * F[6]);
+    if (!(J > 0.0f)) return false;
+    float B[6], ev[3];
+    left_strain(F, B);
+    sym_eig3(B, ev);
+    if (!(ev[2] > -0.99f)) return false;
+    const float e0 = 0.5f * log1pf(ev[0]), e1 = 0.5f * log1pf(ev[1]), e2 = 0.5f * log1pf(ev[2]);
+    const float q0 = 1.0f + ev[0], q1 = 1.0f + ev[1], q2 = 1.0f + ev[2];
+    Newton3 N;
+    newton3_setup(B, ev, N);
+    float T[6];
+    newton3_eval(N, e0, e2, 0.5f * log_ratio_div(q0, q1), 0.5f * log_ratio_div(q1, q2), T);
+    const float dia = lam * (e0 + e1 + e2), tm = 2.0f * mu;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) T[k] = tm * T[k] + ((k == 0 || k == 3 || k == 5) ? dia : 0.0f);
+    sym_full(T, tau);
+    return true;
+}
+
+// p2g_sample_all (mpm_utils.py:353-402).  A particle whose base cell is marked
+// sets F = F_disp + I, takes the stress of that F (FCR for jelly and metal,
+// Drucker-Prager for sand; :368-378) and scatters, per node,
+// w m v + dt (-(m / density) stress grad w) and w m.
+//
+// A warp takes 32 consecutive records.  Each lane prepares its particle (stress
+// and the 17 numbers the scatter needs, in shared memory); then, as in the
+// substep's P2G, three groups of nine lanes take a third of them each: lane
+// (i, j) sums its three z nodes in registers over consecutive particles of one
+// base cell and issues one 16-byte atomic per node when the cell changes.  The
+// records are in the cell order of the last substep and the particles have
+// moved since, so the warp first brings particles of one cell together: the
+// atomics (27 per run) are what bounds the kernel.  Measured on 1M marked
+// particles displaced by an eighth of a cell: 81 us; with
+// an SVD per stress and segmented shuffles over the runs as they lie, 126 us.
+constexpr int kRedWarps = 4;
+constexpr int kRedPay = 5;  // float4 of a particle's scatter data
+__global__ void __launch_bounds__(kRedWarps * 32) reduced_p2g_kernel(const MpmScene *__restrict__ scenes, PState st,
+                                                                     MpmReducedGrid g, int n, float dt,
+                                                                     int *status) {
+    __shared__ float4 pay[kRedWarps][kRedPay][32];
     const MpmScene &S = scenes[0];
     if (!grid_matches(S, g, status)) return;  // the same for every thread
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
+    const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31u);
     const int N = g.n_grid;
-    float gp[3] = {0.5f, 0.5f, 0.5f};
+    const float inv_dx = S.inv_dx;
+    float4 q0, q1, q2, q3;
+    float fx[3] = {1.0f, 1.0f, 1.0f};
     int base[3] = {0, 0, 0};
     bool act = false;
     if (i < n) {
-        record_gp(st, i, S.inv_dx, gp);
+        ldpair(st, i, 0, q0, q1);
+        ldpair(st, i, 1, q2, q3);
+        const float gp[3] = {grid_coord(q0.x, q2.x, inv_dx), grid_coord(q0.y, q2.y, inv_dx),
+                             grid_coord(q0.z, q2.z, inv_dx)};
         bool cell_in = true, stencil_in = true;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -140,6 +182,7 @@ __global__ void __launch_bounds__(256) reduced_p2g_kernel(const MpmScene *__rest
             cell_in = cell_in && t > -1.0f && t < (float)N;
             stencil_in = stencil_in && t > -1.0f && t < (float)(N - 2);
             base[d] = (t > -1.0f && t < (float)N) ? (int)t : 0;
+            fx[d] = __fsub_rn(gp[d], (float)base[d]);
         }
         if (!cell_in) {  // the reference reads the mark array out of bounds here
             atomicOr(status, MPM_ST_OUT_OF_DOMAIN);
@@ -149,93 +192,91 @@ __global__ void __launch_bounds__(256) reduced_p2g_kernel(const MpmScene *__rest
         }
     }
     if (__ballot_sync(0xffffffffu, act) == 0u) return;  // the whole warp leaves together
-    float tau[9], v[3] = {0.f, 0.f, 0.f}, m = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) tau[k] = 0.0f;
+    // the particle's place among the warp's, grouped by cell in the order of the
+    // cells' first lanes (-1: not marked)
+    const int key = act ? ((base[0] << 20) | (base[1] << 10) | base[2]) : -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    const int leader = __ffs(peers) - 1;
+    int at = __popc(peers & ((1u << lane) - 1u));
+    for (unsigned heads = __ballot_sync(0xffffffffu, leader == lane); heads; heads &= heads - 1u) {
+        const int h = __ffs(heads) - 1;
+        const int size = __popc(__shfl_sync(0xffffffffu, peers, h));
+        at += h < leader ? size : 0;
+    }
     if (act) {
-        float4 q1 = ldrec(st, i, 1);
-        const float4 q0 = ldrec(st, i, 0), q2 = ldrec(st, i, 2), q3 = ldrec(st, i, 3);
         const int uid = __float_as_int(q1.y);
         const float *fd = g.f_disp + (int64_t)uid * 9;
-        float F[9];
+        float F[9], tau[9], Fo[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) F[k] = __fadd_rn(fd[k], (k % 4 == 0) ? 1.0f : 0.0f);  // F_disp + I (:364)
-        q1.w = F[8];
-        strec(st, i, 1, q1);
-        strec(st, i, 8, make_float4(F[0], F[1], F[2], F[3]));
-        strec(st, i, 9, make_float4(F[4], F[5], F[6], F[7]));
-        Svd d;
-        svd3(F, d);
-        if (S.material == MPM_SAND) {
-            stress_dp(F, d, S.mu, S.lam, tau);
-        } else {
-            const float J = d.s[0] * d.s[1] * d.s[2];
-            stress_fcr(F, d, J, S.mu, S.lam, tau);
+        stpair(st, i, 0, q0, make_float4(q1.x, q1.y, q1.z, F[8]));
+        stpair(st, i, 4, make_float4(F[0], F[1], F[2], F[3]), make_float4(F[4], F[5], F[6], F[7]));
+        const bool sand = S.material == MPM_SAND;
+        if (!(sand ? stress_dp_spectral(F, S.mu, S.lam, tau) : jelly_stress_spectral(S, F, Fo, tau))) {
+            Svd d;
+            svd3(F, d);
+            if (sand) stress_dp(F, d, S.mu, S.lam, tau);
+            else stress_fcr(F, d, d.s[0] * d.s[1] * d.s[2], S.mu, S.lam, tau);
         }
-        m = q0.w;
-        const float nvol = -__fdiv_rn(m, g.density[uid]);  // -(m / density), :395
-#pragma unroll
-        for (int k = 0; k < 9; ++k) tau[k] *= nvol;
-        v[0] = q2.w;
-        v[1] = q3.x;
-        v[2] = q3.y;
-    } else {  // contributes zeros from a finite stencil
-        gp[0] = gp[1] = gp[2] = 0.5f;
-        base[0] = base[1] = base[2] = 0;
+        const float m = q0.w;
+        const float ts = -__fdiv_rn(m, g.density[uid]) * dt * inv_dx;  // -(m / density) dt / dx, :395
+        pay[warp][0][at] = make_float4(fx[0], fx[1], fx[2], m);
+        pay[warp][1][at] = make_float4(q2.w, q3.x, q3.y,
+                                         __int_as_float(key));
+        pay[warp][2][at] = make_float4(tau[0] * ts, tau[1] * ts, tau[2] * ts, tau[3] * ts);
+        pay[warp][3][at] = make_float4(tau[4] * ts, tau[5] * ts, tau[6] * ts, tau[7] * ts);
+        pay[warp][4][at] = make_float4(tau[8] * ts, 0.0f, 0.0f, 0.0f);
+    } else {
+        pay[warp][1][at] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));  // no cell: skipped
     }
-    // runs of lanes with one base cell (n_grid <= 1024: 10 bits per axis); idle lanes stand alone
-    const int key = act ? ((base[0] << 20) | (base[1] << 10) | base[2]) : (0x40000000 | lane);
-    const int prev = __shfl_up_sync(0xffffffffu, key, 1);
-    const bool head = lane == 0 || prev != key;
-    const unsigned heads = __ballot_sync(0xffffffffu, head);
-    const bool solo = heads == 0xffffffffu;  // no two lanes share a cell: plain atomics
-    // lane + 2^j belongs to this lane's run when no run starts in (lane, lane + 2^j]
-    bool in_run[5];
+    __syncwarp();
+    const int group = lane / 9, ij = lane - 9 * group;
+    if (group >= 3) return;  // lanes 27-31 only prepare (no warp-wide operation follows)
+    const int li = ij / 3, lj = ij - 3 * li;
+    // weight along x: sx (f - cx)^2 + tx, its derivative 2 sx (f - cx); y likewise
+    const float cx = li == 0 ? 1.5f : (li == 1 ? 1.0f : 0.5f), sx = li == 1 ? -1.0f : 0.5f,
+                tx = li == 1 ? 0.75f : 0.0f;
+    const float cy = lj == 0 ? 1.5f : (lj == 1 ? 1.0f : 0.5f), sy = lj == 1 ? -1.0f : 0.5f,
+                ty = lj == 1 ? 0.75f : 0.0f;
+    float4 *grid = static_cast<float4 *>(g.grid_acc);
+    float acc[3][4];
 #pragma unroll
-    for (int j = 0; j < 5; ++j) {
-        const int d = 1 << j;
-        in_run[j] = lane + d < 32 && ((((unsigned long long)heads) >> (lane + 1)) & ((1ull << d) - 1ull)) == 0ull;
-    }
-    Weights W;
-    make_weights(gp, base, W);
-    const float inv_dx = S.inv_dx;
-    float4 *acc = static_cast<float4 *>(g.grid_acc);
+    for (int k = 0; k < 3; ++k) acc[k][0] = acc[k][1] = acc[k][2] = acc[k][3] = 0.0f;
+    int cur = -1;
+    const int last = min(32, 11 * group + 11);
+    for (int p = 11 * group; p <= last; ++p) {
+        const float4 o1 = p < last ? pay[warp][1][p] : make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
+        const int key = __float_as_int(o1.w);
+        if (key != cur && cur >= 0) {
+            float4 *t = grid + dense_index(N, (cur >> 20) + li, ((cur >> 10) & 1023) + lj, cur & 1023);
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            const float wab = W.w[0][a] * W.w[1][b];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const float weight = wab * W.w[2][c];
-                const float dg[3] = {W.dw[0][a] * W.w[1][b] * W.w[2][c] * inv_dx,
-                                     W.w[0][a] * W.dw[1][b] * W.w[2][c] * inv_dx,
-                                     W.w[0][a] * W.w[1][b] * W.dw[2][c] * inv_dx};
-                const float wm = weight * m;
-                float4 add;
-                add.x = wm * v[0] + dt * (tau[0] * dg[0] + tau[1] * dg[1] + tau[2] * dg[2]);
-                add.y = wm * v[1] + dt * (tau[3] * dg[0] + tau[4] * dg[1] + tau[5] * dg[2]);
-                add.z = wm * v[2] + dt * (tau[6] * dg[0] + tau[7] * dg[1] + tau[8] * dg[2]);
-                add.w = wm;
-                if (!solo) {
-#pragma unroll
-                    for (int j = 0; j < 5; ++j) {
-                        const int d = 1 << j;
-                        const float ox = __shfl_down_sync(0xffffffffu, add.x, d);
-                        const float oy = __shfl_down_sync(0xffffffffu, add.y, d);
-                        const float oz = __shfl_down_sync(0xffffffffu, add.z, d);
-                        const float ow = __shfl_down_sync(0xffffffffu, add.w, d);
-                        if (in_run[j]) {
-                            add.x += ox;
-                            add.y += oy;
-                            add.z += oz;
-                            add.w += ow;
-                        }
-                    }
-                }
-                if (act && head) atomicAdd(acc + dense_index(N, base[0] + a, base[1] + b, base[2] + c), add);
+            for (int k = 0; k < 3; ++k) {
+                atomicAdd(t + k, make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]));
+                acc[k][0] = acc[k][1] = acc[k][2] = acc[k][3] = 0.0f;
             }
         }
+        cur = key;
+        if (key < 0) continue;
+        const float4 o0 = pay[warp][0][p], o2 = pay[warp][2][p], o3 = pay[warp][3][p];
+        const float t22 = pay[warp][4][p].x;
+        const float dxi = o0.x - cx, dyj = o0.y - cy;
+        const float ex = sx * dxi, ey = sy * dyj;
+        const float wx = fmaf(ex, dxi, tx), wy = fmaf(ey, dyj, ty);
+        const float za = o0.z - 1.5f, zb = o0.z - 1.0f, zc = o0.z - 0.5f;
+        const float w[3] = {0.5f * za * za, fmaf(-zb, zb, 0.75f), 0.5f * zc * zc};
+        const float dw[3] = {za, -2.0f * zb, zc};
+        const float p1 = 2.0f * ex * wy, p2 = 2.0f * ey * wx, p3 = wx * wy, pm = p3 * o0.w;
+        const float v[3] = {o1.x, o1.y, o1.z};
+        const float t0[3] = {o2.x, o2.w, o3.z}, t1[3] = {o2.y, o3.x, o3.w}, t2[3] = {o2.z, o3.y, t22};
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            const float a = fmaf(pm, v[r], fmaf(t0[r], p1, t1[r] * p2)), d = t2[r] * p3;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) acc[k][r] = fmaf(w[k], a, fmaf(dw[k], d, acc[k][r]));
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) acc[k][3] = fmaf(w[k], pm, acc[k][3]);
+    }
 }
 
 // grid_normalization_and_gravity_sample_all (mpm_utils.py:405-413) fused with
@@ -375,18 +416,26 @@ __global__ void __launch_bounds__(128) g2p_sample_kernel(const MpmScene *__restr
     for (int k = 0; k < 9; ++k) fd[k] = Fn[k] - ((k % 4 == 0) ? 1.0f : 0.0f);  // :471
 }
 
+// zero_grid (both mark arrays and the accumulator) and slot_of_uid, in one launch
+__global__ void __launch_bounds__(256) reduced_clear_kernel(PState st, int n, int *__restrict__ slot_of_uid,
+                                                            MpmReducedGrid g, int64_t nn) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    float4 *acc = static_cast<float4 *>(g.grid_acc);
+    for (int64_t q = i; q < nn; q += stride) acc[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int64_t q = i; q < nn; q += stride) g.neighboring_cells[q] = 0;
+    for (int64_t q = i; q < nn; q += stride) g.neighboring_cells_grid_v[q] = 0;
+    for (int64_t p = i; p < n; p += stride) slot_of_uid[__float_as_int(ldrec(st, (int)p, 1).y)] = (int)p;
+}
+
 cudaError_t launch_p2g2p_reduced(const Ctx &cx, const MpmReducedGrid &g, float time, float dt) {
     const int64_t nn = (int64_t)g.n_grid * g.n_grid * g.n_grid;
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(g.grid_acc, 0, nn * 16, cx.stream)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(g.neighboring_cells, 0, nn * 4, cx.stream)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(g.neighboring_cells_grid_v, 0, nn * 4, cx.stream)) != cudaSuccess) return e;
+    reduced_clear_kernel<<<cx.num_sms * 8, 256, 0, cx.stream>>>(cx.st, cx.n, cx.ws.slot_of_uid, g, nn);
     if (cx.n > 0) {
-        if ((e = launch_slot_of_uid(cx)) != cudaSuccess) return e;
         if (g.n_samples > 0)
             mark_kernel<2><<<(unsigned)((g.n_samples + 7) / 8), 256, 0, cx.stream>>>(
                 cx.scenes, cx.st, cx.ws.slot_of_uid, g, g.neighboring_cells, cx.n, cx.status);
-        reduced_p2g_kernel<<<(cx.n + 255) / 256, 256, 0, cx.stream>>>(cx.scenes, cx.st, g, cx.n, dt, cx.status);
+        reduced_p2g_kernel<<<(cx.n + kRedWarps * 32 - 1) / (kRedWarps * 32), kRedWarps * 32, 0, cx.stream>>>(
+            cx.scenes, cx.st, g, cx.n, dt, cx.status);
     }
     const int64_t want = (nn + 255) / 256;
     const int blocks = (int)(want < (int64_t)cx.num_sms * 16 ? want : (int64_t)cx.num_sms * 16);

@@ -266,3 +266,26 @@ def test_full_size_properties(cuda):
     sb = base[sample.long().to(base.device)]
     for d in (-2, 2):
         assert bool((mask[sb[:, 0] + d, sb[:, 1] + d, sb[:, 2] + d] == 1).all())
+
+
+@pytest.mark.parametrize("material", ["sand", "jelly"])
+@pytest.mark.parametrize("n", [1, 2, 11, 31, 32, 33, 129])
+def test_reduced_scatter_at_warp_edges(cuda, n, material):
+    """The scatter's grouping by cell where the lanes' cells are in no order
+    (records as loaded), in crowded and single cells, marked and not; jelly also
+    with inverted elements (the SVD stress)."""
+    sc, sim, ref = _pair(material, n=n, n_grid=12, steps=0, n_samples=1)
+    rng = np.random.default_rng(n)
+    F = np.eye(3) + 0.05 * rng.normal(size=(n, 3, 3))
+    if material == "jelly":
+        F[::3, 0] *= -1.0
+    fd = (F - np.eye(3)).astype(np.float32)
+    u = (0.02 * rng.normal(size=(n, 3))).astype(np.float32)
+    v = rng.normal(size=(n, 3)).astype(np.float32)
+    sim.load_uvF_from_tensor(torch.from_numpy(u), torch.from_numpy(v), torch.from_numpy(fd))
+    for r in (ref, ref.twin):
+        r.u[:], r.v[:], r.F_disp[:] = u, v, fd.reshape(n, 9)
+    for _ in range(2):  # nothing moves: the same grid again, from cleared arrays
+        _reduced(sim, ref, sc.dt)
+        _check_grid(sim, ref)
+    assert np.array_equal(gpu_state(sim)["F"], ref.F)
