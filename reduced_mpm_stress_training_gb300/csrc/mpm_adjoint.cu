@@ -32,6 +32,7 @@
 namespace mpm {
 namespace adj {
 
+constexpr int kThreads = 128;  // of the two particle kernels
 constexpr int kAdjWords = 36;
 enum { AX = 0, AV = 3, AC = 6, AF = 15, AT = 24 };
 
@@ -268,25 +269,25 @@ struct NodeW {
     float H[3][3];   // Hessian wrt x
 };
 
-__device__ __forceinline__ void node_weights(const Weights &W, int i, int j, int k, float inv_dx, NodeW &o) {
-    const int nd[3] = {i, j, k};
-    float a[3], da[3], dda[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        a[d] = W.w[d][nd[d]];
-        da[d] = W.dw[d][nd[d]] * inv_dx;
-        dda[d] = ddw(nd[d]) * inv_dx * inv_dx;
-    }
-    o.w = a[0] * a[1] * a[2];
-    o.dw[0] = da[0] * a[1] * a[2];
-    o.dw[1] = a[0] * da[1] * a[2];
-    o.dw[2] = a[0] * a[1] * da[2];
-    o.H[0][0] = dda[0] * a[1] * a[2];
-    o.H[1][1] = a[0] * dda[1] * a[2];
-    o.H[2][2] = a[0] * a[1] * dda[2];
-    o.H[0][1] = o.H[1][0] = da[0] * da[1] * a[2];
-    o.H[0][2] = o.H[2][0] = da[0] * a[1] * da[2];
-    o.H[1][2] = o.H[2][1] = a[0] * da[1] * da[2];
+// entry i of a register array, by selects (a run-time index would put it in local memory)
+__device__ __forceinline__ float plane(const float (&a)[3], int i) { return i == 0 ? a[0] : (i == 1 ? a[1] : a[2]); }
+
+// weight, gradient and Hessian of node (i, j, k), given the x factors of i
+__device__ __forceinline__ void node_weights(const Weights &W, float ax, float dax, float ddax, int j, int k,
+                                             float inv_dx, NodeW &o) {
+    const float ay = W.w[1][j], az = W.w[2][k];
+    const float day = W.dw[1][j] * inv_dx, daz = W.dw[2][k] * inv_dx;
+    const float dday = ddw(j) * inv_dx * inv_dx, ddaz = ddw(k) * inv_dx * inv_dx;
+    o.w = ax * ay * az;
+    o.dw[0] = dax * ay * az;
+    o.dw[1] = ax * day * az;
+    o.dw[2] = ax * ay * daz;
+    o.H[0][0] = ddax * ay * az;
+    o.H[1][1] = ax * dday * az;
+    o.H[2][2] = ax * ay * ddaz;
+    o.H[0][1] = o.H[1][0] = dax * day * az;
+    o.H[0][2] = o.H[2][0] = dax * ay * daz;
+    o.H[1][2] = o.H[2][1] = ax * day * daz;
 }
 
 struct PData {
@@ -308,23 +309,51 @@ __device__ __forceinline__ void particle_stencil(const MpmScene &S, const float 
     p.ok = ok;
 }
 
+// quad q of an adjoint record, whole (vec: the caller's buffer is 16-byte aligned) or by words
+__device__ __forceinline__ float4 ldadj(const float *a, int q, bool vec) {
+    if (vec) return reinterpret_cast<const float4 *>(a)[q];
+    return make_float4(a[q * 4], a[q * 4 + 1], a[q * 4 + 2], a[q * 4 + 3]);
+}
+__device__ __forceinline__ void stadj(float *a, int q, float x, float y, float z, float w, bool vec) {
+    if (vec) {
+        reinterpret_cast<float4 *>(a)[q] = make_float4(x, y, z, w);
+    } else {
+        a[q * 4] = x;
+        a[q * 4 + 1] = y;
+        a[q * 4 + 2] = z;
+        a[q * 4 + 3] = w;
+    }
+}
+
+__device__ __forceinline__ void load_F(const PState &st, int slot, float (&F)[9]) {
+    const float4 a = ldrec(st, slot, rec::F0 / 4), b = ldrec(st, slot, rec::F0 / 4 + 1);
+    F[0] = a.x; F[1] = a.y; F[2] = a.z; F[3] = a.w;
+    F[4] = b.x; F[5] = b.y; F[6] = b.z; F[7] = b.w;
+    F[8] = recword(st, slot, rec::F8);
+}
+
 // ---------------------------------------------------------------------------
-// G2P adjoint: thread per sorted position.
+// G2P adjoint: thread per sorted position.  Bound by instruction issue and
+// fetch at few warps an SM (28 M instructions, 46 % of the issue slots; DRAM 7 %),
+// so the code and the registers were cut: both node loops run a plane at a time
+// (27 copies of each body waited for instructions), the scatter reads the
+// velocities again instead of holding 81 registers since the gather, and F, the
+// position and the weights are made again after the return map.  255 registers
+// and spills at 2 blocks an SM -> 128 at 4: 82 -> 62 us at 131k particles (gather
+// unrolled 64; 168 registers at 3 blocks 65; 96 at 5, 72; blocks of 64 threads 64).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) g2p_adjoint_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
+__global__ void __launch_bounds__(kThreads, 4) g2p_adjoint_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
                                                           PState st, Ws ws, const float *__restrict__ adj_out,
                                                           float *__restrict__ adj_in,
                                                           float4 *__restrict__ grid_adj, double *__restrict__ thb_out,
-                                                          float dt) {
+                                                          float dt, bool vec) {
     float thb[3] = {0.0f, 0.0f, 0.0f};
     for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < ws.n; pos += gridDim.x * blockDim.x) {
         const int slot = ws.order[pos];
-        // the record quads this kernel reads (x0 | uid, F8 | u | F0-7), as
-        // 16-byte loads; w indexes them by record word
-        float4 rq[kRecQuads];
+        // record quads 0-2 (x0 | uid, F8 | u) as 16-byte loads; w indexes them by record word
+        float4 rq[3];
 #pragma unroll
-        for (int q = 0; q < kRecQuads; ++q)
-            rq[q] = (q < 3 || q >= 8) ? ldrec(st, slot, q) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int q = 0; q < 3; ++q) rq[q] = ldrec(st, slot, q);
         const float *w = reinterpret_cast<const float *>(rq);
         const int uid = __float_as_int(w[rec::UID]);
         const MpmScene &S = scenes[scene_of_particle(scenes, n_scenes, uid)];
@@ -344,32 +373,27 @@ __global__ void __launch_bounds__(128) g2p_adjoint_kernel(const MpmScene *__rest
         make_weights(p.gp, p.base, W);
         const float inv_dx = S.inv_dx;
         const int nb = S.n_blocks_axis;
-        // forward recompute: nv, nF (velocity gradient), F_trial
-        float gv[27][3];
-        float nv[3] = {0.f, 0.f, 0.f}, nF[9] = {0.f};
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
+        // forward recompute: nF (velocity gradient), F_trial
+        float nF[9] = {0.f};
+#pragma unroll 1
+        for (int i = 0; i < 3; ++i) {
+            const float ax = plane(W.w[0], i), dax = plane(W.dw[0], i) * inv_dx;
 #pragma unroll
             for (int j = 0; j < 3; ++j)
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    const int q = (i * 3 + j) * 3 + k;
                     const float4 g4 = ws.grid_v[node_addr(S.block_begin, nb, p.base[0] + i, p.base[1] + j, p.base[2] + k)];
-                    gv[q][0] = g4.x; gv[q][1] = g4.y; gv[q][2] = g4.z;
+                    const float g[3] = {g4.x, g4.y, g4.z};
                     NodeW nw;
-                    node_weights(W, i, j, k, inv_dx, nw);
+                    node_weights(W, ax, dax, 0.0f, j, k, inv_dx, nw);
 #pragma unroll
-                    for (int r = 0; r < 3; ++r) {
-                        nv[r] += gv[q][r] * nw.w;
+                    for (int r = 0; r < 3; ++r)
 #pragma unroll
-                        for (int c = 0; c < 3; ++c) nF[r * 3 + c] += gv[q][r] * nw.dw[c];
-                    }
+                        for (int c = 0; c < 3; ++c) nF[r * 3 + c] += g[r] * nw.dw[c];
                 }
-        float Fo[9];
-        Fo[0] = w[rec::F0 + 0]; Fo[1] = w[rec::F0 + 1]; Fo[2] = w[rec::F0 + 2]; Fo[3] = w[rec::F0 + 3];
-        Fo[4] = w[rec::F0 + 4]; Fo[5] = w[rec::F0 + 5]; Fo[6] = w[rec::F0 + 6]; Fo[7] = w[rec::F0 + 7];
-        Fo[8] = w[rec::F8];
-        float A[9], Ft[9];
+        }
+        float A[9], Ft[9], Fo[9];
+        load_F(st, slot, Fo);
 #pragma unroll
         for (int q = 0; q < 9; ++q) A[q] = ((q % 4 == 0) ? 1.0f : 0.0f) + nF[q] * dt;
 #pragma unroll
@@ -379,42 +403,71 @@ __global__ void __launch_bounds__(128) g2p_adjoint_kernel(const MpmScene *__rest
                 Ft[r * 3 + c] = A[r * 3 + 0] * Fo[0 * 3 + c] + A[r * 3 + 1] * Fo[1 * 3 + c] + A[r * 3 + 2] * Fo[2 * 3 + c];
         // return map adjoint
         float Fb[9], Tb[9], Ftb[9];
+        {
+            float4 t4[6];  // words 12-35: C's last three, F, stress
 #pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            Fb[q] = ao[AF + q];
-            Tb[q] = ao[AT + q];
-            Ftb[q] = 0.0f;
+            for (int q = 0; q < 6; ++q) t4[q] = ldadj(ao, q + 3, vec);
+            const float *t = reinterpret_cast<const float *>(t4);
+#pragma unroll
+            for (int q = 0; q < 9; ++q) {
+                Fb[q] = t[AF - 12 + q];
+                Tb[q] = t[AT - 12 + q];
+                Ftb[q] = 0.0f;
+            }
         }
         sand_rm_vjp(S, Ft, Fb, Tb, Ftb, thb);
+        // F, the position and the weights again, behind a slot number that the compiler
+        // can't tell from a new one: not held across the return map's SVD
+        int again = slot;
+        asm volatile("" : "+r"(again) : "f"(Ftb[0]));
+        load_F(st, again, Fo);
+        rq[0] = ldrec(st, again, 0);
+        rq[2] = ldrec(st, again, 2);
+        particle_stencil(S, w, p);
+        make_weights(p.gp, p.base, W);
         // F_trial = A F: F_old adjoint A^T Ftb; nF adjoint dt Ftb F^T
-        float nFb[9];
+        float nFb[9], Fob[9];
 #pragma unroll
         for (int r = 0; r < 3; ++r)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                ai[AF + r * 3 + c] = A[0 * 3 + r] * Ftb[0 * 3 + c] + A[1 * 3 + r] * Ftb[1 * 3 + c] + A[2 * 3 + r] * Ftb[2 * 3 + c];
+                Fob[r * 3 + c] = A[0 * 3 + r] * Ftb[0 * 3 + c] + A[1 * 3 + r] * Ftb[1 * 3 + c] + A[2 * 3 + r] * Ftb[2 * 3 + c];
                 nFb[r * 3 + c] = dt * (Ftb[r * 3 + 0] * Fo[c * 3 + 0] + Ftb[r * 3 + 1] * Fo[c * 3 + 1] + Ftb[r * 3 + 2] * Fo[c * 3 + 2]);
             }
+        // words 12-23 (the P2G adjoint writes C's words 12-14)
+        stadj(ai, 3, 0.0f, 0.0f, 0.0f, Fob[0], vec);
+        stadj(ai, 4, Fob[1], Fob[2], Fob[3], Fob[4], vec);
+        stadj(ai, 5, Fob[5], Fob[6], Fob[7], Fob[8], vec);
         float nvb[3], nCb[9], xb[3];
+        {
+            float4 t4[4];  // words 0-15: x, v, C
 #pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            xb[r] = ao[AX + r];
-            nvb[r] = ao[AV + r] + dt * ao[AX + r];  // x' = x + dt v', v' = nv
+            for (int q = 0; q < 4; ++q) t4[q] = ldadj(ao, q, vec);
+            const float *t = reinterpret_cast<const float *>(t4);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                xb[r] = t[AX + r];
+                nvb[r] = t[AV + r] + dt * t[AX + r];  // x' = x + dt v', v' = nv
+            }
+#pragma unroll
+            for (int q = 0; q < 9; ++q) nCb[q] = t[AC + q];
         }
-#pragma unroll
-        for (int q = 0; q < 9; ++q) nCb[q] = ao[AC + q];
         const float c4 = 4.0f * inv_dx;
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
+#pragma unroll 1
+        for (int i = 0; i < 3; ++i) {
+            const float ax = plane(W.w[0], i), dax = plane(W.dw[0], i) * inv_dx;
+            const float ddax = ddw(i) * inv_dx * inv_dx;
+            const float dpx = (float)i - W.fx[0];
 #pragma unroll
             for (int j = 0; j < 3; ++j)
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    const int q = (i * 3 + j) * 3 + k;
+                    const int64_t at = node_addr(S.block_begin, nb, p.base[0] + i, p.base[1] + j, p.base[2] + k);
+                    const float4 g4 = ws.grid_v[at];
+                    const float g[3] = {g4.x, g4.y, g4.z};
                     NodeW nw;
-                    node_weights(W, i, j, k, inv_dx, nw);
-                    const float dpos[3] = {(float)i - W.fx[0], (float)j - W.fx[1], (float)k - W.fx[2]};
-                    const float *g = gv[q];
+                    node_weights(W, ax, dax, ddax, j, k, inv_dx, nw);
+                    const float dpos[3] = {dpx, (float)j - W.fx[1], (float)k - W.fx[2]};
                     // node adjoint: nv += g w, nC += g dpos^T (4 inv_dx w), nF += g dw^T
                     float gb[3];
 #pragma unroll
@@ -424,8 +477,7 @@ __global__ void __launch_bounds__(128) g2p_adjoint_kernel(const MpmScene *__rest
                                 nFb[r * 3 + 0] * nw.dw[0] + nFb[r * 3 + 1] * nw.dw[1] + nFb[r * 3 + 2] * nw.dw[2];
                     }
                     // one vector atomic per node (w, unused until the grid adjoint overwrites it, gets 0)
-                    atomicAdd(grid_adj + node_addr(S.block_begin, nb, p.base[0] + i, p.base[1] + j, p.base[2] + k),
-                              make_float4(gb[0], gb[1], gb[2], 0.0f));
+                    atomicAdd(grid_adj + at, make_float4(gb[0], gb[1], gb[2], 0.0f));
                     // particle position adjoint through the weights and dpos
                     const float gvb = nvb[0] * g[0] + nvb[1] * g[1] + nvb[2] * g[2];
                     float qv[3], sv[3];
@@ -440,8 +492,8 @@ __global__ void __launch_bounds__(128) g2p_adjoint_kernel(const MpmScene *__rest
                         xb[d] += gvb * nw.dw[d] + c4 * (qd * nw.dw[d] - qv[d] * inv_dx * nw.w) +
                                  sv[0] * nw.H[0][d] + sv[1] * nw.H[1][d] + sv[2] * nw.H[2][d];
                 }
-#pragma unroll
-        for (int d = 0; d < 3; ++d) ai[AX + d] = xb[d];  // v, C and stress adjoints: written by the P2G adjoint
+        }
+        stadj(ai, 0, xb[0], xb[1], xb[2], 0.0f, vec);  // v, C and stress adjoints: written by the P2G adjoint
     }
     // parameter adjoints: warp sums, one double atomic per warp and parameter
 #pragma unroll
@@ -514,11 +566,15 @@ __global__ void __launch_bounds__(256) grid_adjoint_kernel(const MpmScene *__res
 }
 
 // ---------------------------------------------------------------------------
-// P2G adjoint: thread per sorted position; gathers the node adjoints.
+// P2G adjoint: thread per sorted position; gathers the node adjoints.  The 27
+// loads stay unrolled, all in flight at once (a plane at a time took 80 us:
+// bound by their latency).  Adjoint records move as 16-byte quads, 8 accesses
+// and 4 words a particle where single words were 27: 33 -> 25 us at 131k
+// particles (128 registers at 4 blocks an SM: the same, with spills).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) p2g_adjoint_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
+__global__ void __launch_bounds__(kThreads, 3) p2g_adjoint_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
                                                           PState st, Ws ws, const float4 *__restrict__ grid_adj,
-                                                          float *__restrict__ adj_in, float dt) {
+                                                          float *__restrict__ adj_in, float dt, bool vec) {
     for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < ws.n; pos += gridDim.x * blockDim.x) {
         const int slot = ws.order[pos];
         // record quads 0-7 (x0, m | vol, uid | u, v | C | tau) as 16-byte loads
@@ -546,16 +602,18 @@ __global__ void __launch_bounds__(128) p2g_adjoint_kernel(const MpmScene *__rest
         }
         float vb[3] = {0.f, 0.f, 0.f}, Cb[9] = {0.f}, Tb[9] = {0.f}, xb[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
+        for (int i = 0; i < 3; ++i) {
+            const float ax = W.w[0][i], dax = W.dw[0][i] * inv_dx, ddax = ddw(i) * inv_dx * inv_dx;
+            const float dpx = ((float)i - W.fx[0]) * dx;
 #pragma unroll
             for (int j = 0; j < 3; ++j)
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     NodeW nw;
-                    node_weights(W, i, j, k, inv_dx, nw);
+                    node_weights(W, ax, dax, ddax, j, k, inv_dx, nw);
                     const float4 g = grid_adj[node_addr(S.block_begin, nb, p.base[0] + i, p.base[1] + j, p.base[2] + k)];
                     const float mvb[3] = {g.x, g.y, g.z};
-                    const float dpos[3] = {((float)i - W.fx[0]) * dx, ((float)j - W.fx[1]) * dx, ((float)k - W.fx[2]) * dx};
+                    const float dpos[3] = {dpx, ((float)j - W.fx[1]) * dx, ((float)k - W.fx[2]) * dx};
                     float mom[3];  // m (v + C dpos)
 #pragma unroll
                     for (int r = 0; r < 3; ++r)
@@ -582,17 +640,18 @@ __global__ void __launch_bounds__(128) p2g_adjoint_kernel(const MpmScene *__rest
                         xb[d] += s0 * nw.dw[d] - wm * ctm[d] -
                                  dt * vol * (ttm[0] * nw.H[0][d] + ttm[1] * nw.H[1][d] + ttm[2] * nw.H[2][d]);
                 }
+        }
         float *ai = adj_in + (int64_t)uid * kAdjWords;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            ai[AX + d] += xb[d];
-            ai[AV + d] = vb[d];
-        }
-#pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            ai[AC + q] = Cb[q];
-            ai[AT + q] = Tb[q];
-        }
+        const float4 x4 = ldadj(ai, 0, vec);
+        stadj(ai, 0, x4.x + xb[0], x4.y + xb[1], x4.z + xb[2], vb[0], vec);
+        stadj(ai, 1, vb[1], vb[2], Cb[0], Cb[1], vec);
+        stadj(ai, 2, Cb[2], Cb[3], Cb[4], Cb[5], vec);
+        ai[12] = Cb[6];
+        ai[13] = Cb[7];
+        ai[14] = Cb[8];
+        stadj(ai, 6, Tb[0], Tb[1], Tb[2], Tb[3], vec);
+        stadj(ai, 7, Tb[4], Tb[5], Tb[6], Tb[7], vec);
+        ai[32] = Tb[8];
     }
 }
 
@@ -643,16 +702,20 @@ cudaError_t launch_return_map_vjp(const MpmScene &scene, const float *Ft, const 
 cudaError_t launch_adjoint(const Ctx &cx, const float *adj_out, float *adj_in, float4 *grid_adj, double *thb,
                            float time, float dt) {
     using namespace adj;
-    const int pgrid = (int)((cx.n + 127) / 128 < (int64_t)cx.num_sms * 8 ? (cx.n + 127) / 128 : cx.num_sms * 8);
+    const int64_t want = (cx.n + kThreads - 1) / kThreads;
+    const int pgrid = (int)(want < (int64_t)cx.num_sms * 8 ? want : (int64_t)cx.num_sms * 8);
     const int ggrid = (int)((cx.total_blocks + 3) / 4 < (int64_t)cx.num_sms * 8 ? (cx.total_blocks + 3) / 4
                                                                                 : cx.num_sms * 8);
     if (cx.n <= 0) return cudaSuccess;
+    // 16-byte accesses where both buffers allow them (a caller's view may start at any word)
+    const bool vec = ((reinterpret_cast<uintptr_t>(adj_out) | reinterpret_cast<uintptr_t>(adj_in)) & 15) == 0;
     zero_active_kernel<<<cx.num_sms * 4, 256, 0, cx.stream>>>(cx.ws, grid_adj);
-    g2p_adjoint_kernel<<<pgrid, 128, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.st, cx.ws, adj_out, adj_in,
-                                                     grid_adj, thb, dt);
+    g2p_adjoint_kernel<<<pgrid, kThreads, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.st, cx.ws, adj_out, adj_in,
+                                                     grid_adj, thb, dt, vec);
     grid_adjoint_kernel<<<ggrid > 0 ? ggrid : 1, 256, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.ws, grid_adj,
                                                                       time, dt);
-    p2g_adjoint_kernel<<<pgrid, 128, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.st, cx.ws, grid_adj, adj_in, dt);
+    p2g_adjoint_kernel<<<pgrid, kThreads, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.st, cx.ws, grid_adj, adj_in, dt,
+                                                        vec);
     return cudaGetLastError();
 }
 
