@@ -347,6 +347,7 @@ __global__ void __launch_bounds__(kThreads, 4) g2p_adjoint_kernel(const MpmScene
                                                           float *__restrict__ adj_in,
                                                           float4 *__restrict__ grid_adj, double *__restrict__ thb_out,
                                                           float dt, bool vec) {
+    chain_wait();
     float thb[3] = {0.0f, 0.0f, 0.0f};
     for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < ws.n; pos += gridDim.x * blockDim.x) {
         const int slot = ws.order[pos];
@@ -512,6 +513,7 @@ __global__ void __launch_bounds__(kThreads, 4) g2p_adjoint_kernel(const MpmScene
 __global__ void __launch_bounds__(256) grid_adjoint_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
                                                            Ws ws, float4 *__restrict__ grid_adj, float time,
                                                            float dt) {
+    chain_wait();
     const int n_active = *ws.n_active;
     const int l = threadIdx.x & 63;
     for (int base = blockIdx.x * 4; base < n_active; base += gridDim.x * 4) {
@@ -575,6 +577,7 @@ __global__ void __launch_bounds__(256) grid_adjoint_kernel(const MpmScene *__res
 __global__ void __launch_bounds__(kThreads, 3) p2g_adjoint_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
                                                           PState st, Ws ws, const float4 *__restrict__ grid_adj,
                                                           float *__restrict__ adj_in, float dt, bool vec) {
+    chain_wait();
     for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < ws.n; pos += gridDim.x * blockDim.x) {
         const int slot = ws.order[pos];
         // record quads 0-7 (x0, m | vol, uid | u, v | C | tau) as 16-byte loads
@@ -657,6 +660,7 @@ __global__ void __launch_bounds__(kThreads, 3) p2g_adjoint_kernel(const MpmScene
 
 // zero the adjoint of the substep's active grid blocks
 __global__ void zero_active_kernel(Ws ws, float4 *__restrict__ grid_adj) {
+    chain_wait();
     const int n_active = *ws.n_active;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_active * kBlockNodes; i += gridDim.x * blockDim.x)
         grid_adj[(int64_t)ws.active_list[i / kBlockNodes] * kBlockNodes + i % kBlockNodes] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -709,12 +713,15 @@ cudaError_t launch_adjoint(const Ctx &cx, const float *adj_out, float *adj_in, f
     if (cx.n <= 0) return cudaSuccess;
     // 16-byte accesses where both buffers allow them (a caller's view may start at any word)
     const bool vec = ((reinterpret_cast<uintptr_t>(adj_out) | reinterpret_cast<uintptr_t>(adj_in)) & 15) == 0;
-    zero_active_kernel<<<cx.num_sms * 4, 256, 0, cx.stream>>>(cx.ws, grid_adj);
-    g2p_adjoint_kernel<<<pgrid, kThreads, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.st, cx.ws, adj_out, adj_in,
+    launch_chained(zero_active_kernel, cx.num_sms * 4, 256, 0, cx.stream, cx.ws, grid_adj);
+    launch_chained(g2p_adjoint_kernel, pgrid, kThreads, 0, cx.stream, cx.scenes, cx.n_scenes, cx.st, cx.ws, adj_out,
+                   adj_in,
                                                      grid_adj, thb, dt, vec);
-    grid_adjoint_kernel<<<ggrid > 0 ? ggrid : 1, 256, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.ws, grid_adj,
+    launch_chained(grid_adjoint_kernel, ggrid > 0 ? ggrid : 1, 256, 0, cx.stream, cx.scenes, cx.n_scenes, cx.ws,
+                   grid_adj,
                                                                       time, dt);
-    p2g_adjoint_kernel<<<pgrid, kThreads, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.st, cx.ws, grid_adj, adj_in, dt,
+    launch_chained(p2g_adjoint_kernel, pgrid, kThreads, 0, cx.stream, cx.scenes, cx.n_scenes, cx.st, cx.ws, grid_adj,
+                   adj_in, dt,
                                                         vec);
     return cudaGetLastError();
 }

@@ -50,6 +50,7 @@ inline Blob blob_view(void *base, int64_t total_blocks, int64_t n, int64_t max_c
 // Counts and the active-block list are read from the side being copied from.
 template <bool SAVE>
 __global__ void blob_kernel(Ws ws, Blob b, int n) {
+    chain_wait();
     const int na = SAVE ? *ws.n_active : *b.n_active;
     const int nc = min(SAVE ? *ws.n_chunks : *b.n_chunks, ws.max_chunks);
     const int *list = SAVE ? ws.active_list : b.list;
@@ -99,14 +100,14 @@ int64_t substep_grid_bytes(int64_t total_blocks, int64_t n, int64_t max_chunks) 
 cudaError_t launch_save_grid(const Ctx &cx, void *dst) {
     using namespace ckpt;
     Blob b = blob_view(dst, cx.total_blocks, cx.n, cx.ws.max_chunks);
-    blob_kernel<true><<<cx.num_sms * 8, 256, 0, cx.stream>>>(cx.ws, b, (int)cx.n);
+    launch_chained(blob_kernel<true>, cx.num_sms * 8, 256, 0, cx.stream, cx.ws, b, (int)cx.n);
     return cudaGetLastError();
 }
 
 cudaError_t launch_load_grid(const Ctx &cx, const void *src) {
     using namespace ckpt;
     Blob b = blob_view(const_cast<void *>(src), cx.total_blocks, cx.n, cx.ws.max_chunks);
-    blob_kernel<false><<<cx.num_sms * 8, 256, 0, cx.stream>>>(cx.ws, b, (int)cx.n);
+    launch_chained(blob_kernel<false>, cx.num_sms * 8, 256, 0, cx.stream, cx.ws, b, (int)cx.n);
     return cudaGetLastError();
 }
 

@@ -223,6 +223,7 @@ template <int HP>
 __global__ void __launch_bounds__(kDecThreads) decoder_stress_kernel(MpmStressDecoder d, PState st,
                                                                      const float *__restrict__ label,
                                                                      const float *__restrict__ mu, int n) {
+    chain_wait();
     extern __shared__ float4 sm4[];
     float *sm = reinterpret_cast<float *>(sm4);
     const int L0 = d.label_dim, M = d.mu_dim, in = L0 + 3 + M;
@@ -429,6 +430,7 @@ __global__ void __launch_bounds__(P * dtc::kRows, P == 2 ? 3 : 4) decoder_stress
                                                                           const float *__restrict__ label,
                                                                           const float *__restrict__ mu, int n,
                                                                           int *status) {
+    chain_wait();
     using namespace dtc;
     extern __shared__ __align__(128) unsigned char dtc_smem_raw[];
     Smem<P> &s = *reinterpret_cast<Smem<P> *>(dtc_smem_raw);
@@ -632,11 +634,11 @@ cudaError_t launch_decoder_stress(const Ctx &cx, const MpmStressDecoder &d, cons
         const int tiles = (cx.n + dtc::kRows - 1) / dtc::kRows;
         const int groups = (tiles + P - 1) / P;
         const int tgrid = groups < cx.num_sms * per_sm ? groups : cx.num_sms * per_sm;
-        decoder_stress_tc_kernel<P><<<tgrid, P * dtc::kRows, bytes, cx.stream>>>(d, cx.st, label, mu, cx.n,
+        launch_chained(decoder_stress_tc_kernel<P>, tgrid, P * dtc::kRows, bytes, cx.stream, d, cx.st, label, mu, cx.n,
                                                                                  cx.status);
     } else {
         if ((e = dec_prepare(decoder_stress_kernel<64>, 3)) != cudaSuccess) return e;
-        decoder_stress_kernel<64><<<grid, kDecThreads, smem, cx.stream>>>(d, cx.st, label, mu, cx.n);
+        launch_chained(decoder_stress_kernel<64>, grid, kDecThreads, smem, cx.stream, d, cx.st, label, mu, cx.n);
     }
     return cudaGetLastError();
 }

@@ -51,6 +51,7 @@ __global__ void init_state_kernel(PState a, PState b, int n) {
 }
 
 __global__ void load_kernel(PState st, int n, int field, int nc, const float *__restrict__ src) {
+    chain_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int64_t u = __float_as_int(recword(st, i, rec::UID));
@@ -64,6 +65,7 @@ __global__ void load_kernel(PState st, int n, int field, int nc, const float *__
 // stresses: 54 -> 22 us.
 template <int NC>
 __global__ void __launch_bounds__(256) export_kernel(PState st, int n, int field, float *__restrict__ dst) {
+    chain_wait();
     __shared__ float rows[8][32 * NC];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = (int)(threadIdx.x & 31u);
@@ -95,6 +97,7 @@ __global__ void __launch_bounds__(256) export_kernel(PState st, int n, int field
 // sectors) -- scattering 12- and 36-byte rows by uid instead leaves partial
 // sectors that L2 cannot merge once the arrays outgrow it
 __global__ void slot_of_uid_kernel(PState st, int n, int *__restrict__ inv) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     inv[__float_as_int(ldrec(st, i, 1).y)] = i;
@@ -102,7 +105,8 @@ __global__ void slot_of_uid_kernel(PState st, int n, int *__restrict__ inv) {
 
 cudaError_t launch_slot_of_uid(const Ctx &cx) {
     if (cx.n == 0) return cudaSuccess;
-    slot_of_uid_kernel<<<(unsigned)((cx.n + 255) / 256), 256, 0, cx.stream>>>(cx.st, cx.n, cx.ws.slot_of_uid);
+    launch_chained(slot_of_uid_kernel, (unsigned)((cx.n + 255) / 256), 256, 0, cx.stream, cx.st, cx.n,
+                   cx.ws.slot_of_uid);
     return cudaGetLastError();
 }
 
@@ -111,6 +115,7 @@ cudaError_t launch_slot_of_uid(const Ctx &cx) {
 // words sharing quads 3 and 5 are kept)
 __global__ void load_uvstress_kernel(PState st, int n, const int *__restrict__ inv, const float *__restrict__ u,
                                      const float *__restrict__ v, const float *__restrict__ tau) {
+    chain_wait();
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= n) return;
     const int i = inv[id];
@@ -130,6 +135,7 @@ constexpr int kExportWarps = 4;
 __global__ void __launch_bounds__(kExportWarps * 32) export_uvFstress_kernel(
     PState st, int n, const int *__restrict__ inv, float *__restrict__ u, float *__restrict__ v,
     float *__restrict__ fd, float *__restrict__ tau) {
+    chain_wait();
     __shared__ float rows[kExportWarps][32 * 24];  // u, v, F - I, stress of 32 particles
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = (int)(threadIdx.x & 31u);
@@ -179,6 +185,7 @@ __global__ void __launch_bounds__(kExportWarps * 32) export_uvFstress_kernel(
 // f_tensor = F - I (9, n) | stress components 0,1,2,4,5,8 (6, n) | v (3, n) |
 // C (9, n).
 __global__ void export_frame_kernel(PState st, int n, const int *__restrict__ inv, float *__restrict__ out) {
+    chain_wait();
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= n) return;
     const int i = inv[id];
@@ -270,7 +277,7 @@ cudaError_t launch_init_state(const Ctx &cx, const PState &other) {
 
 cudaError_t launch_load(const Ctx &cx, int field, const float *src) {
     if (cx.n == 0) return cudaSuccess;
-    load_kernel<<<blocks_for(cx.n, 256), 256, 0, cx.stream>>>(cx.st, cx.n, field,
+    launch_chained(load_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, field,
                                                                field_components(field), src);
     return cudaGetLastError();
 }
@@ -279,32 +286,33 @@ cudaError_t launch_export(const Ctx &cx, int field, float *dst) {
     if (cx.n == 0) return cudaSuccess;
     const unsigned grid = blocks_for(cx.n, 256);
     switch (field_components(field)) {
-        case 1: export_kernel<1><<<grid, 256, 0, cx.stream>>>(cx.st, cx.n, field, dst); break;
-        case 3: export_kernel<3><<<grid, 256, 0, cx.stream>>>(cx.st, cx.n, field, dst); break;
-        default: export_kernel<9><<<grid, 256, 0, cx.stream>>>(cx.st, cx.n, field, dst); break;
+        case 1: launch_chained(export_kernel<1>, grid, 256, 0, cx.stream, cx.st, cx.n, field, dst); break;
+        case 3: launch_chained(export_kernel<3>, grid, 256, 0, cx.stream, cx.st, cx.n, field, dst); break;
+        default: launch_chained(export_kernel<9>, grid, 256, 0, cx.stream, cx.st, cx.n, field, dst); break;
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_load_uvstress(const Ctx &cx, const float *u, const float *v, const float *tau) {
     if (cx.n == 0) return cudaSuccess;
-    slot_of_uid_kernel<<<blocks_for(cx.n, 256), 256, 0, cx.stream>>>(cx.st, cx.n, cx.ws.slot_of_uid);
-    load_uvstress_kernel<<<blocks_for(cx.n, 256), 256, 0, cx.stream>>>(cx.st, cx.n, cx.ws.slot_of_uid, u, v, tau);
+    launch_chained(slot_of_uid_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid);
+    launch_chained(load_uvstress_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid, u,
+                   v, tau);
     return cudaGetLastError();
 }
 
 cudaError_t launch_export_uvFstress(const Ctx &cx, float *u, float *v, float *fd, float *tau) {
     if (cx.n == 0) return cudaSuccess;
-    slot_of_uid_kernel<<<blocks_for(cx.n, 256), 256, 0, cx.stream>>>(cx.st, cx.n, cx.ws.slot_of_uid);
-    export_uvFstress_kernel<<<blocks_for(cx.n, kExportWarps * 32), kExportWarps * 32, 0, cx.stream>>>(
+    launch_chained(slot_of_uid_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid);
+    launch_chained(export_uvFstress_kernel, blocks_for(cx.n, kExportWarps * 32), kExportWarps * 32, 0, cx.stream,
         cx.st, cx.n, cx.ws.slot_of_uid, u, v, fd, tau);
     return cudaGetLastError();
 }
 
 cudaError_t launch_export_frame(const Ctx &cx, float *out) {
     if (cx.n == 0) return cudaSuccess;
-    slot_of_uid_kernel<<<blocks_for(cx.n, 256), 256, 0, cx.stream>>>(cx.st, cx.n, cx.ws.slot_of_uid);
-    export_frame_kernel<<<blocks_for(cx.n, 256), 256, 0, cx.stream>>>(cx.st, cx.n, cx.ws.slot_of_uid, out);
+    launch_chained(slot_of_uid_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid);
+    launch_chained(export_frame_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid, out);
     return cudaGetLastError();
 }
 

@@ -32,6 +32,29 @@ cudaError_t launch_p2g(const Ctx &cx, float dt);
 // node in a fixed order into grid_acc.  scratch: ordered_scratch_bytes
 int64_t ordered_scratch_bytes(int64_t total_blocks);
 cudaError_t launch_p2g_ordered(const Ctx &cx, float dt, void *scratch);
+// Starts a kernel whose first statement is chain_wait() (programmatic dependent
+// launch): its launch and its blocks' start overlap the tail of the kernel before it
+// in the stream, which saves the gap of about 2 us that an ordinary launch leaves
+// (eager substep of 32k particles 39.1 -> 25.8 us, 300k 88.1 -> 74.2, 1M 178 -> 166;
+// in a graph, where the gaps are shorter, 26.6 -> 24.8, 75.0 -> 72.5, 164 -> 164).
+// No kernel says launch_dependents itself: blocks of the next kernel that wait for it
+// all the while take the place of its own, and P2G's next wave (32k in a graph 29.4).
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), int64_t grid, int block, size_t smem, cudaStream_t stream,
+                           A... args) {
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 cudaError_t launch_grid(const Ctx &cx, float time, float dt);
 // kFast: the substep's form; kPinned: results that do not change from build to
 // build (the stage entry point and the ordered mode); kDeferStress: store

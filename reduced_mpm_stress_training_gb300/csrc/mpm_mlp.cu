@@ -90,6 +90,7 @@ __device__ __forceinline__ void a1_from_x(uint32_t a1[1][4], const float *x, int
 
 __global__ void __launch_bounds__(256) mlp_forward_kernel(const __nv_bfloat16 *__restrict__ w,
                                                           const float *__restrict__ b, FwdIO io) {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char mlp_smem[];
     WSmem &s = *reinterpret_cast<WSmem *>(mlp_smem);
     load_weights(s, w, b);
@@ -113,6 +114,7 @@ __global__ void __launch_bounds__(128) mlp_dgrad_kernel(const __nv_bfloat16 *__r
                                                         const __nv_bfloat16 *__restrict__ wnext,
                                                         const __nv_bfloat16 *__restrict__ z,
                                                         __nv_bfloat16 *__restrict__ dz, int64_t n) {
+    chain_wait();
     constexpr int LDA = NN + 8;
     extern __shared__ __align__(16) unsigned char mlp_smem[];
     __nv_bfloat16 *ws = reinterpret_cast<__nv_bfloat16 *>(mlp_smem);  // [NN][LDW]
@@ -176,6 +178,7 @@ __global__ void __launch_bounds__(128) mlp_wgrad_kernel(const __nv_bfloat16 *__r
                                                         const __nv_bfloat16 *__restrict__ zp,
                                                         const float *__restrict__ x, float *__restrict__ dw,
                                                         float *__restrict__ db, int64_t n, int rows_per_cta) {
+    chain_wait();
     constexpr int LDD = NO + 8, LDH = KI + 8, RT = 32;  // rows staged per step
     __shared__ __align__(16) __nv_bfloat16 ds[RT * LDD];
     __shared__ __align__(16) __nv_bfloat16 hs[RT * LDH];
@@ -270,6 +273,7 @@ __global__ void mlp_adam_kernel(float *__restrict__ master, float *__restrict__ 
                                 const float *__restrict__ grad, __nv_bfloat16 *__restrict__ wbf,
                                 float *__restrict__ bias, int count, float lr, float b1, float b2,
                                 float eps, float c1, float c2) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     bool pad = false;
@@ -356,7 +360,8 @@ int mpm_mlp_forward(const void *params, const float *x, float *y, const float *t
     const float *b = reinterpret_cast<const float *>(static_cast<const char *>(params) + (int64_t)W_COUNT * 2);
     FwdIO io{x, y, target, static_cast<__nv_bfloat16 *>(zsave), static_cast<__nv_bfloat16 *>(dy), loss,
              grad_scale, n};
-    mlp_forward_kernel<<<mlp_grid((n + 15) / 16, 8, 1), 256, sizeof(WSmem), static_cast<cudaStream_t>(stream)>>>(
+    mpm::launch_chained(mlp_forward_kernel, mlp_grid((n + 15) / 16, 8, 1), 256, sizeof(WSmem),
+                        static_cast<cudaStream_t>(stream),
         w, b, io);
     return cudaGetLastError() == cudaSuccess ? MPM_OK : MPM_ERR_CUDA;
 }
@@ -383,16 +388,21 @@ int mpm_mlp_backward(const void *params, const float *x, const void *zsave, cons
     const int gridd = mlp_grid((n + 15) / 16, 4, 4);
     const __nv_bfloat16 *dyb = static_cast<const __nv_bfloat16 *>(dy);
     // layer 4: dW4 += dY^T H3, dZ3 = (dY W4) * silu'(Z3)
-    mlp_wgrad_kernel<N4, H, false><<<gridw, 128, 0, st>>>(dyb, z + 2 * n * H, nullptr, gw + W4_OFF, gb + B4_OFF, n, rows);
-    mlp_dgrad_kernel<N4><<<gridd, 128, dgrad_smem<N4>(), st>>>(dyb, w + W4_OFF, z + 2 * n * H, dz3, n);
+    mpm::launch_chained(mlp_wgrad_kernel<N4, H, false>, gridw, 128, 0, st, dyb, z + 2 * n * H, nullptr, gw + W4_OFF,
+                        gb + B4_OFF, n, rows);
+    mpm::launch_chained(mlp_dgrad_kernel<N4>, gridd, 128, dgrad_smem<N4>(), st, dyb, w + W4_OFF, z + 2 * n * H, dz3,
+                        n);
     // layer 3
-    mlp_wgrad_kernel<H, H, false><<<gridw, 128, 0, st>>>(dz3, z + 1 * n * H, nullptr, gw + W3_OFF, gb + B3_OFF, n, rows);
-    mlp_dgrad_kernel<H><<<gridd, 128, dgrad_smem<H>(), st>>>(dz3, w + W3_OFF, z + 1 * n * H, dz2, n);
+    mpm::launch_chained(mlp_wgrad_kernel<H, H, false>, gridw, 128, 0, st, dz3, z + 1 * n * H, nullptr, gw + W3_OFF,
+                        gb + B3_OFF, n, rows);
+    mpm::launch_chained(mlp_dgrad_kernel<H>, gridd, 128, dgrad_smem<H>(), st, dz3, w + W3_OFF, z + 1 * n * H, dz2, n);
     // layer 2
-    mlp_wgrad_kernel<H, H, false><<<gridw, 128, 0, st>>>(dz2, z + 0 * n * H, nullptr, gw + W2_OFF, gb + B2_OFF, n, rows);
-    mlp_dgrad_kernel<H><<<gridd, 128, dgrad_smem<H>(), st>>>(dz2, w + W2_OFF, z + 0 * n * H, dz3, n);
+    mpm::launch_chained(mlp_wgrad_kernel<H, H, false>, gridw, 128, 0, st, dz2, z + 0 * n * H, nullptr, gw + W2_OFF,
+                        gb + B2_OFF, n, rows);
+    mpm::launch_chained(mlp_dgrad_kernel<H>, gridd, 128, dgrad_smem<H>(), st, dz2, w + W2_OFF, z + 0 * n * H, dz3, n);
     // layer 1: dW1 += dZ1^T X
-    mlp_wgrad_kernel<H, K1, true><<<gridw, 128, 0, st>>>(dz3, nullptr, x, gw + W1_OFF, gb + B1_OFF, n, rows);
+    mpm::launch_chained(mlp_wgrad_kernel<H, K1, true>, gridw, 128, 0, st, dz3, nullptr, x, gw + W1_OFF, gb + B1_OFF,
+                        n, rows);
     return cudaGetLastError() == cudaSuccess ? MPM_OK : MPM_ERR_CUDA;
 }
 
@@ -404,7 +414,7 @@ int mpm_mlp_adam(float *master, float *m, float *v, const float *grad, void *par
     const float c2 = 1.0f / (1.0f - powf(beta2, (float)step));
     __nv_bfloat16 *wbf = static_cast<__nv_bfloat16 *>(params);
     float *bias = reinterpret_cast<float *>(static_cast<char *>(params) + (int64_t)W_COUNT * 2);
-    mlp_adam_kernel<<<(count + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    mpm::launch_chained(mlp_adam_kernel, (count + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream),
         master, m, v, grad, wbf, bias, count, lr, beta1, beta2, eps, c1, c2);
     return cudaGetLastError() == cudaSuccess ? MPM_OK : MPM_ERR_CUDA;
 }

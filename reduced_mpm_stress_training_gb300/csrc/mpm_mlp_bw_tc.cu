@@ -177,6 +177,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) mlp_backward_tc_kernel(const __
                                                                      const __nv_bfloat16 *__restrict__ dy,
                                                                      float *__restrict__ grad, int64_t n,
                                                                      int *__restrict__ err) {
+    chain_wait();
     extern __shared__ __align__(128) unsigned char bw_smem_raw[];
     BwSmem &s = *reinterpret_cast<BwSmem *>(bw_smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -409,7 +410,8 @@ cudaError_t launch_mlp_backward_tc(const void *params, const float *x, const voi
     const int64_t tiles = (n + kRows - 1) / kRows;
     // one CTA per SM (each holds all 512 tensor-memory columns)
     const int grid = (int)(tiles < (int64_t)num_sms ? tiles : (int64_t)num_sms);
-    mlp_backward_tc_kernel<<<grid, kBwThreads, bytes, stream>>>(w, x, static_cast<const __nv_bfloat16 *>(zsave),
+    launch_chained(mlp_backward_tc_kernel, grid, kBwThreads, bytes, stream, w, x,
+                   static_cast<const __nv_bfloat16 *>(zsave),
                                                               static_cast<const __nv_bfloat16 *>(dy), grad, n, err);
     return cudaGetLastError();
 }

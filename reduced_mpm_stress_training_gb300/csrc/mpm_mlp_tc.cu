@@ -146,6 +146,7 @@ __device__ __forceinline__ void load_x(const TcIO &io, int64_t row, float (&v)[I
 __global__ void __launch_bounds__(kFwThreads, 1) mlp_forward_tc_kernel(const __nv_bfloat16 *__restrict__ w,
                                                                        const float *__restrict__ b, TcIO io,
                                                                        int *__restrict__ err) {
+    chain_wait();
     extern __shared__ __align__(128) unsigned char tc_smem_raw[];
     FwSmem &s = *reinterpret_cast<FwSmem *>(tc_smem_raw);
     const int pipe = (int)threadIdx.x / kThreads, tid = (int)threadIdx.x % kThreads, warp = tid >> 5;
@@ -317,7 +318,7 @@ cudaError_t launch_mlp_forward_tc(const void *params, const float *x, float *y, 
     const int64_t tiles = (n + kRows - 1) / kRows;
     // small batches spread over the SMs before they fill a CTA's pipelines
     const int grid = (int)(tiles < (int64_t)num_sms ? tiles : (int64_t)num_sms);
-    mlp_forward_tc_kernel<<<grid, kFwThreads, bytes, stream>>>(w, b, io, err);
+    launch_chained(mlp_forward_tc_kernel, grid, kFwThreads, bytes, stream, w, b, io, err);
     return cudaGetLastError();
 }
 

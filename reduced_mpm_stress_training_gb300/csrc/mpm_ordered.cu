@@ -38,6 +38,7 @@ __device__ __forceinline__ int rec_uid(const PState &st, int slot) {
 // of order[] by uid.  Cells hold a handful of particles; the sort is
 // quadratic in the cell's count.
 __global__ void __launch_bounds__(256) canonical_cells_kernel(PState st, Ws ws) {
+    chain_wait();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int bi = (int)(t >> 6), c = (int)(t & 63);
     if (bi >= *ws.n_blocks) return;
@@ -292,6 +293,7 @@ __device__ __forceinline__ bool p2g_next_round(int &rem0, int &rem1, int &pos0, 
 __global__ void __launch_bounds__(32, 2) p2g_tiles_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
                                                           PState st, Ws ws, float dt, int *status,
                                                           float4 *partials, int *blk_index) {
+    chain_wait();
     __shared__ P2GWarpSmem sm;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -404,6 +406,7 @@ __global__ void __launch_bounds__(32, 2) p2g_tiles_kernel(const MpmScene *__rest
 __global__ void __launch_bounds__(256) gather_partials_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
                                                               Ws ws, const float4 *__restrict__ partials,
                                                               const int *__restrict__ blk_index) {
+    chain_wait();
     const int n_active = *ws.n_active;
     const int l = threadIdx.x & 63;
     for (int base = blockIdx.x * 4; base < n_active; base += gridDim.x * 4) {
@@ -449,19 +452,21 @@ cudaError_t launch_p2g_ordered(const Ctx &cx, float dt, void *scratch) {
     if (e != cudaSuccess) return e;
     const int64_t threads = cx.total_blocks * 64;
     if (threads > 0) {
-        canonical_cells_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, cx.stream>>>(cx.st, cx.ws);
+        launch_chained(canonical_cells_kernel, (unsigned)((threads + 255) / 256), 256, 0, cx.stream, cx.st, cx.ws);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     // up to 32 single-warp CTAs per SM, several times the resident ones: the
     // rest start as others finish, which balances blocks of unequal size
     const int64_t tw = cx.total_blocks < (int64_t)cx.num_sms * 32 ? cx.total_blocks : (int64_t)cx.num_sms * 32;
-    p2g_tiles_kernel<<<(unsigned)(tw > 0 ? tw : 1), 32, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.st, cx.ws, dt,
+    launch_chained(p2g_tiles_kernel, (unsigned)(tw > 0 ? tw : 1), 32, 0, cx.stream, cx.scenes, cx.n_scenes, cx.st,
+                   cx.ws, dt,
                                                                         cx.status, partials, blk_index);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int64_t want = (cx.total_blocks + 3) / 4;
     int grid = (int)(want < (int64_t)cx.num_sms * 8 ? want : (int64_t)cx.num_sms * 8);
     if (grid < 1) grid = 1;
-    gather_partials_kernel<<<grid, 256, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.ws, partials, blk_index);
+    launch_chained(gather_partials_kernel, grid, 256, 0, cx.stream, cx.scenes, cx.n_scenes, cx.ws, partials,
+                   blk_index);
     return cudaGetLastError();
 }
 

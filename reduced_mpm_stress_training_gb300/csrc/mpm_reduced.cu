@@ -82,6 +82,7 @@ template <int HI>
 __global__ void __launch_bounds__(256) mark_kernel(const MpmScene *__restrict__ scenes, PState st,
                                                    const int *__restrict__ slot_of_uid, MpmReducedGrid g,
                                                    int32_t *__restrict__ mask, int n, int *status) {
+    chain_wait();
     const MpmScene &S = scenes[0];
     if (!grid_matches(S, g, status)) return;
     const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -159,6 +160,7 @@ constexpr int kRedPay = 5;  // float4 of a particle's scatter data
 __global__ void __launch_bounds__(kRedWarps * 32) reduced_p2g_kernel(const MpmScene *__restrict__ scenes, PState st,
                                                                      MpmReducedGrid g, int n, float dt,
                                                                      int *status) {
+    chain_wait();
     __shared__ float4 pay[kRedWarps][kRedPay][32];
     const MpmScene &S = scenes[0];
     if (!grid_matches(S, g, status)) return;  // the same for every thread
@@ -286,6 +288,7 @@ __global__ void __launch_bounds__(kRedWarps * 32) reduced_p2g_kernel(const MpmSc
 // collider in registration order, over every node.
 __global__ void __launch_bounds__(256) reduced_grid_kernel(const MpmScene *__restrict__ scenes, MpmReducedGrid g,
                                                            float time, float dt, int *status) {
+    chain_wait();
     const MpmScene &S = scenes[0];
     if (!grid_matches(S, g, status)) return;
     const int N = g.n_grid;
@@ -320,6 +323,7 @@ __global__ void __launch_bounds__(256) reduced_grid_kernel(const MpmScene *__res
 __global__ void __launch_bounds__(128) g2p_sample_kernel(const MpmScene *__restrict__ scenes, PState st,
                                                          const int *__restrict__ slot_of_uid, MpmReducedGrid g,
                                                          int n, float dt, int *status) {
+    chain_wait();
     const MpmScene &S = scenes[0];
     if (!grid_matches(S, g, status)) return;
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -419,6 +423,7 @@ __global__ void __launch_bounds__(128) g2p_sample_kernel(const MpmScene *__restr
 // zero_grid (both mark arrays and the accumulator) and slot_of_uid, in one launch
 __global__ void __launch_bounds__(256) reduced_clear_kernel(PState st, int n, int *__restrict__ slot_of_uid,
                                                             MpmReducedGrid g, int64_t nn) {
+    chain_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
     float4 *acc = static_cast<float4 *>(g.grid_acc);
     for (int64_t q = i; q < nn; q += stride) acc[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -429,17 +434,17 @@ __global__ void __launch_bounds__(256) reduced_clear_kernel(PState st, int n, in
 
 cudaError_t launch_p2g2p_reduced(const Ctx &cx, const MpmReducedGrid &g, float time, float dt) {
     const int64_t nn = (int64_t)g.n_grid * g.n_grid * g.n_grid;
-    reduced_clear_kernel<<<cx.num_sms * 8, 256, 0, cx.stream>>>(cx.st, cx.n, cx.ws.slot_of_uid, g, nn);
+    launch_chained(reduced_clear_kernel, cx.num_sms * 8, 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid, g, nn);
     if (cx.n > 0) {
         if (g.n_samples > 0)
-            mark_kernel<2><<<(unsigned)((g.n_samples + 7) / 8), 256, 0, cx.stream>>>(
-                cx.scenes, cx.st, cx.ws.slot_of_uid, g, g.neighboring_cells, cx.n, cx.status);
-        reduced_p2g_kernel<<<(cx.n + kRedWarps * 32 - 1) / (kRedWarps * 32), kRedWarps * 32, 0, cx.stream>>>(
-            cx.scenes, cx.st, g, cx.n, dt, cx.status);
+            launch_chained(mark_kernel<2>, (unsigned)((g.n_samples + 7) / 8), 256, 0, cx.stream, cx.scenes, cx.st,
+                           cx.ws.slot_of_uid, g, g.neighboring_cells, cx.n, cx.status);
+        launch_chained(reduced_p2g_kernel, (cx.n + kRedWarps * 32 - 1) / (kRedWarps * 32), kRedWarps * 32, 0,
+                       cx.stream, cx.scenes, cx.st, g, cx.n, dt, cx.status);
     }
     const int64_t want = (nn + 255) / 256;
     const int blocks = (int)(want < (int64_t)cx.num_sms * 16 ? want : (int64_t)cx.num_sms * 16);
-    reduced_grid_kernel<<<blocks > 0 ? blocks : 1, 256, 0, cx.stream>>>(cx.scenes, g, time, dt, cx.status);
+    launch_chained(reduced_grid_kernel, blocks > 0 ? blocks : 1, 256, 0, cx.stream, cx.scenes, g, time, dt, cx.status);
     return cudaGetLastError();
 }
 
@@ -447,8 +452,8 @@ cudaError_t launch_mark_grid_v(const Ctx &cx, const MpmReducedGrid &g) {
     if (cx.n == 0 || g.n_samples == 0) return cudaSuccess;
     cudaError_t e = launch_slot_of_uid(cx);
     if (e != cudaSuccess) return e;
-    mark_kernel<4><<<(unsigned)((g.n_samples + 7) / 8), 256, 0, cx.stream>>>(
-        cx.scenes, cx.st, cx.ws.slot_of_uid, g, g.neighboring_cells_grid_v, cx.n, cx.status);
+    launch_chained(mark_kernel<4>, (unsigned)((g.n_samples + 7) / 8), 256, 0, cx.stream, cx.scenes, cx.st,
+                   cx.ws.slot_of_uid, g, g.neighboring_cells_grid_v, cx.n, cx.status);
     return cudaGetLastError();
 }
 
@@ -456,8 +461,8 @@ cudaError_t launch_g2p_sample(const Ctx &cx, const MpmReducedGrid &g, float dt) 
     if (cx.n == 0 || g.n_samples == 0) return cudaSuccess;
     cudaError_t e = launch_slot_of_uid(cx);
     if (e != cudaSuccess) return e;
-    g2p_sample_kernel<<<(unsigned)((g.n_samples + 127) / 128), 128, 0, cx.stream>>>(
-        cx.scenes, cx.st, cx.ws.slot_of_uid, g, cx.n, dt, cx.status);
+    launch_chained(g2p_sample_kernel, (unsigned)((g.n_samples + 127) / 128), 128, 0, cx.stream, cx.scenes, cx.st,
+                   cx.ws.slot_of_uid, g, cx.n, dt, cx.status);
     return cudaGetLastError();
 }
 

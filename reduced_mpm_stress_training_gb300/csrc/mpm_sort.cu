@@ -25,6 +25,7 @@ namespace mpm {
 // keys + histogram straight from x0 + u (used after loads)
 __global__ void key_kernel(const MpmScene *__restrict__ scenes, int n_scenes, PState st, Ws ws,
                            int n, int *status) {
+    chain_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int key = -1;
     if (i < n) {
@@ -94,6 +95,7 @@ __device__ __forceinline__ int4 cta_sum4(int4 v, int4 *wsum /* [kScanWarps] shar
 // the counts themselves.
 constexpr int kSumTile = 512;
 __global__ void __launch_bounds__(kScanThreads) bucket_sums_kernel(Ws ws) {
+    chain_wait();
     __shared__ int4 wsum[kScanWarps];
     int4 acc = make_int4(0, 0, 0, 0);
 #pragma unroll
@@ -126,6 +128,7 @@ constexpr int kWideBuckets = 1 << 17;
 template <bool SUMS, int KB>
 __global__ void __launch_bounds__(kScanThreads) scan_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
                                                             Ws ws) {
+    chain_wait();
     __shared__ int4 wsum[kScanWarps];
     __shared__ int s_off[KB], s_coff[KB], s_boff[KB], s_cnt[KB];
     __shared__ int s_list[KB];
@@ -237,6 +240,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const MpmScene *__re
 constexpr int kScatterPer = 4;
 
 __global__ void __launch_bounds__(256) scatter_kernel(PState st, Ws ws, int n) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int stride = gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
@@ -271,7 +275,7 @@ __global__ void __launch_bounds__(256) scatter_kernel(PState st, Ws ws, int n) {
 
 cudaError_t launch_keys(const Ctx &cx) {
     if (cx.n == 0) return cudaSuccess;
-    key_kernel<<<(cx.n + 255) / 256, 256, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.st, cx.ws,
+    launch_chained(key_kernel, (cx.n + 255) / 256, 256, 0, cx.stream, cx.scenes, cx.n_scenes, cx.st, cx.ws,
                                                            cx.n, cx.status);
     return cudaGetLastError();
 }
@@ -279,13 +283,16 @@ cudaError_t launch_keys(const Ctx &cx) {
 cudaError_t launch_sort(const Ctx &cx) {
     const int nbk = cx.ws.nbk;
     if (nbk <= kDirectBuckets) {
-        scan_kernel<false, 64><<<(nbk + 63) / 64, kScanThreads, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.ws);
+        launch_chained(scan_kernel<false, 64>, (nbk + 63) / 64, kScanThreads, 0, cx.stream, cx.scenes, cx.n_scenes,
+                       cx.ws);
     } else {
-        bucket_sums_kernel<<<(nbk + kSumTile - 1) / kSumTile, kScanThreads, 0, cx.stream>>>(cx.ws);
+        launch_chained(bucket_sums_kernel, (nbk + kSumTile - 1) / kSumTile, kScanThreads, 0, cx.stream, cx.ws);
         if (nbk <= kWideBuckets)
-            scan_kernel<true, 64><<<(nbk + 63) / 64, kScanThreads, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.ws);
+            launch_chained(scan_kernel<true, 64>, (nbk + 63) / 64, kScanThreads, 0, cx.stream, cx.scenes,
+                           cx.n_scenes, cx.ws);
         else
-            scan_kernel<true, 256><<<(nbk + 255) / 256, kScanThreads, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.ws);
+            launch_chained(scan_kernel<true, 256>, (nbk + 255) / 256, kScanThreads, 0, cx.stream, cx.scenes,
+                           cx.n_scenes, cx.ws);
     }
     // kScatterPer keys a thread, but never fewer than two CTAs an SM: the blocks to
     // clear do not shrink with the particles (a few CTAs clearing a sparse scene's
@@ -294,7 +301,7 @@ cudaError_t launch_sort(const Ctx &cx) {
     const int per = 256 * kScatterPer;
     int sgrid = (cx.n + per - 1) / per;
     if (sgrid < 2 * cx.num_sms) sgrid = 2 * cx.num_sms;
-    scatter_kernel<<<sgrid, 256, 0, cx.stream>>>(cx.st, cx.ws, cx.n);
+    launch_chained(scatter_kernel, sgrid, 256, 0, cx.stream, cx.st, cx.ws, cx.n);
     return cudaGetLastError();
 }
 

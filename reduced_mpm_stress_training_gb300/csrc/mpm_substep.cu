@@ -163,6 +163,7 @@ __device__ __forceinline__ void p2g_flush(float4 *mytile, int cell, unsigned gma
 __global__ void __launch_bounds__(kP2GWarps * 32, 6) p2g_kernel(const MpmScene *__restrict__ scenes,
                                                                 int n_scenes, PState st, Ws ws, float dt,
                                                                 int *status) {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char p2g_smem_raw[];
     P2GSmem &sm = *reinterpret_cast<P2GSmem *>(p2g_smem_raw);
     const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -313,6 +314,7 @@ __global__ void advance_colliders_kernel(MpmScene *__restrict__ scenes, int n_sc
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) grid_kernel(const MpmScene *__restrict__ scenes,
                                                    int n_scenes, Ws ws, float time, float dt) {
+    chain_wait();
     const int n_active = *ws.n_active;
     const int l = threadIdx.x & 63;
     for (int base = blockIdx.x * 4; base < n_active; base += gridDim.x * 4) {
@@ -462,6 +464,7 @@ __device__ __forceinline__ int g2p_slot(const Ws &ws, const int4 &ch) {
 template <int CH, bool DEFER, bool FAST>
 __global__ void __launch_bounds__(CH, FAST ? 640 / CH : 0) g2p_kernel(const MpmScene *__restrict__ scenes, PState st,
                                                  PState out, Ws ws, float dt, int *status) {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char g2p_smem_raw[];
     G2PSmem<CH> &sm = *reinterpret_cast<G2PSmem<CH> *>(g2p_smem_raw);
     const int n_chunks = *ws.n_chunks;
@@ -708,7 +711,8 @@ static cudaError_t g2p_t(const Ctx &cx, float dt) {
         resident[dev] = nb > 0 ? nb : 1;
     }
     const int grid = persistent_grid(cx, resident[dev]);
-    g2p_kernel<CH, DEFER, FAST><<<grid, CH, bytes, cx.stream>>>(cx.scenes, cx.st, cx.st2, cx.ws, dt, cx.status);
+    launch_chained(g2p_kernel<CH, DEFER, FAST>, grid, CH, bytes, cx.stream, cx.scenes, cx.st, cx.st2, cx.ws, dt,
+                   cx.status);
     return cudaGetLastError();
 }
 
@@ -720,8 +724,8 @@ cudaError_t launch_p2g(const Ctx &cx, float dt) {
     // blocks when there are more blocks than CTAs
     int grid = (int)(cx.total_blocks < (int64_t)cx.num_sms * 24 ? cx.total_blocks : (int64_t)cx.num_sms * 24);
     if (grid < 1) grid = 1;
-    p2g_kernel<<<grid, kP2GWarps * 32, bytes, cx.stream>>>(cx.scenes, cx.n_scenes, cx.st, cx.ws, dt,
-                                                           cx.status);
+    launch_chained(p2g_kernel, grid, kP2GWarps * 32, bytes, cx.stream, cx.scenes, cx.n_scenes, cx.st, cx.ws, dt,
+                   cx.status);
     return cudaGetLastError();
 }
 
@@ -729,7 +733,7 @@ cudaError_t launch_grid(const Ctx &cx, float time, float dt) {
     int64_t want = (cx.total_blocks + 3) / 4;
     int grid = (int)(want < (int64_t)cx.num_sms * 8 ? want : (int64_t)cx.num_sms * 8);
     if (grid < 1) grid = 1;
-    grid_kernel<<<grid, 256, 0, cx.stream>>>(cx.scenes, cx.n_scenes, cx.ws, time, dt);
+    launch_chained(grid_kernel, grid, 256, 0, cx.stream, cx.scenes, cx.n_scenes, cx.ws, time, dt);
     return cudaGetLastError();
 }
 

@@ -387,6 +387,7 @@ __global__ void __launch_bounds__(mlptc::kThreads, 2)
     surrogate_tc_kernel(const MpmScene *__restrict__ scenes, PState st, Ws ws, const __nv_bfloat16 *__restrict__ wts,
                         const float *__restrict__ bias, MpmSurrogateConfig cfg, int2 *__restrict__ fallback,
                         int *__restrict__ stats, int *__restrict__ status) {
+    chain_wait();
     extern __shared__ __align__(128) unsigned char tc_raw[];
     mlptc::TcSmem &s = *reinterpret_cast<mlptc::TcSmem *>(tc_raw);
     const int tid = threadIdx.x, lane = tid & 31;
@@ -467,6 +468,7 @@ __global__ void __launch_bounds__(mlptc::kThreads, 2)
 // SVD return map for the listed particles (the exact path)
 __global__ void fallback_kernel(const MpmScene *__restrict__ scenes, PState st, const int2 *__restrict__ list,
                                 const int *__restrict__ stats, int *__restrict__ status) {
+    chain_wait();
     const int n = stats[MPM_SUR_LAST_FALLBACKS];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int2 e = list[i];
@@ -520,14 +522,15 @@ cudaError_t launch_surrogate(const Ctx &cx, const void *mlp_params, const MpmSur
     const int64_t items = (int64_t)cx.ws.max_chunks * ((cx.ws.chunk_size + kTcRows - 1) / kTcRows);
     int grid = (int)(items < 2 * (int64_t)cx.num_sms ? items : 2 * (int64_t)cx.num_sms);
     if (grid < 1) grid = 1;
-    surrogate_tc_kernel<<<grid, mlptc::kThreads, bytes, cx.stream>>>(cx.scenes, cx.st2, cx.ws, w, b, cfg, fallback, stats,
+    launch_chained(surrogate_tc_kernel, grid, mlptc::kThreads, bytes, cx.stream, cx.scenes, cx.st2, cx.ws, w, b, cfg,
+                   fallback, stats,
                                                              cx.status);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     int fgrid = cx.num_sms * 4;
     const int64_t fwant = ((int64_t)cx.n + 127) / 128;
     if (fwant < fgrid) fgrid = (int)(fwant > 0 ? fwant : 1);
-    fallback_kernel<<<fgrid, 128, 0, cx.stream>>>(cx.scenes, cx.st2, fallback, stats, cx.status);
+    launch_chained(fallback_kernel, fgrid, 128, 0, cx.stream, cx.scenes, cx.st2, fallback, stats, cx.status);
     return cudaGetLastError();
 }
 
