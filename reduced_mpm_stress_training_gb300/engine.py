@@ -215,6 +215,18 @@ def _stream_handle(device: torch.device) -> int:
     return torch._C._cuda_getCurrentRawStream(index)
 
 
+_STATUS_STREAMS: dict = {}  # device index -> stream: one a device, since PyTorch's streams are a pool of 32
+
+
+def _status_stream(device: torch.device) -> "torch.cuda.Stream":
+    """The device's stream for reading status words (high priority: not one of those
+    that torch.cuda.Stream() hands to programs by default)."""
+    index = torch.cuda.current_device() if device.index is None else device.index
+    if index not in _STATUS_STREAMS:
+        _STATUS_STREAMS.setdefault(index, torch.cuda.Stream(index, priority=-1))
+    return _STATUS_STREAMS[index]
+
+
 class MPMEngine:
     """Device buffers + C-ABI driver for one or more scenes (concatenated)."""
 
@@ -263,6 +275,7 @@ class MPMEngine:
                 self._status = torch.zeros(1, dtype=torch.int32, device=dev)
                 self._status_host = torch.zeros(1, dtype=torch.int32).pin_memory()
                 self._status_event = torch.cuda.Event()
+                self._status_stream = _status_stream(dev)  # now: making a stream may wait for the device
             self._workspace = torch.zeros(plan.workspace_bytes, dtype=torch.uint8, device=dev)
             self._scenes_dev = torch.empty(C.sizeof(A.MpmScene) * len(self.scenes),
                                            dtype=torch.uint8, device=dev)
@@ -496,6 +509,8 @@ class MPMEngine:
     def reinit(self) -> None:
         """Back to the freshly initialised state (mpm_init: zero state, F = I,
         identity order); the caller reloads the particle fields."""
+        if self._pending and not self._status_copied:
+            self._copy_status()  # mpm_init clears the word: keep what poll_status has yet to read
         A.check(self.lib.mpm_init(C.byref(self.buf), self.stream), "mpm_init")
 
     def snapshot(self) -> tuple:
@@ -519,11 +534,26 @@ class MPMEngine:
         status word is copied to the host behind it; a GPU that has not reached
         the previous mark yet is spared the copy (its kernels would wait about 8 us
         for it), and poll_status reads the word itself once it has caught up."""
-        self._status_copied = not self._pending
-        if self._status_copied:
-            self._status_host.copy_(self._status, non_blocking=True)
+        if self._pending:
+            self._status_copied = False
+            self._status_event.record(torch.cuda.current_stream(self.device))
+        else:
+            self._copy_status()
+
+    def _copy_status(self) -> None:
+        """Queue the status word's copy to the host on the current stream, and mark its end."""
+        self._status_host.copy_(self._status, non_blocking=True)
         self._status_event.record(torch.cuda.current_stream(self.device))
+        self._status_copied = True
         self._pending = True
+
+    def _read_status(self) -> None:
+        """The status word to the host on the device's side stream: the substep is over
+        (its event has passed), so this waits for the copy alone, and not for what
+        else has been queued on the current stream since."""
+        with torch.cuda.stream(self._status_stream):
+            self._status_host.copy_(self._status, non_blocking=True)
+        self._status_stream.synchronize()
 
     def poll_status(self, wait: bool = False) -> int:
         """Read the status word after the last substep (lazy; no sync
@@ -533,8 +563,10 @@ class MPMEngine:
         if not wait and not self._status_event.query():
             return 0
         self._status_event.synchronize()
+        if not self._status_copied:
+            self._read_status()
         self._pending = False
-        bits = int(self._status_host.item()) if self._status_copied else int(self._status.item())
+        bits = int(self._status_host.item())
         if bits:
             self._status.zero_()
             if self.on_error == "raise":
