@@ -627,6 +627,18 @@ __device__ __forceinline__ bool metal_return_map_spectral(const MpmScene &S, con
     return true;
 }
 
+// True where a closed-form stress is at least as close to 64 bits as one from the
+// SVD.  The error of the eigenvalues of B is about 2^-24 max(1, s0^2) in absolute
+// terms and counts relative to the smallest square singular value, s2^2: it grows with
+// the square of the strain, the SVD's with s0 / s2.  Measured on random rotations,
+// median error of the Drucker-Prager stress (closed form, SVD): s = 1.8 to 0.55
+// (max(1, s0^2) = 11 s2^2) 3.1e-7, 4.3e-7; 1 to 0.5 (4) 1.6e-7, 3.0e-7; 0.4 to 0.3 (11)
+// 2.5e-7, 1.7e-7; 2.24 to 0.45 (25) 7.0e-7, 3.8e-7; 5 to 0.2 (625) 4.3e-5, 1.1e-6.
+// The fixed-corotated stress: 1 to 0.5 1.1e-7, 2.8e-7; 0.4 to 0.3 4.4e-7, 1.7e-7.
+__device__ __forceinline__ bool spectral_as_accurate(const float ev[3]) {
+    return fmaxf(1.0f, 1.0f + ev[0]) <= 8.0f * (1.0f + ev[2]);
+}
+
 // ---------------------------------------------------------------------------
 // Fixed-corotated stress without an SVD (kirchoff_stress_FCR,
 // engine_stress/mpm_utils.py:29-34, jelly, F = F_trial):
@@ -634,7 +646,9 @@ __device__ __forceinline__ bool metal_return_map_spectral(const MpmScene &S, con
 // and (F - R) F^T = b - b^{1/2} = f(B), f(beta) = (1 + beta) - sqrt(1 + beta)
 // = sqrt(1 + beta) beta / (1 + sqrt(1 + beta)),  f[x, y] = 1 - 1 / (sqrt(1 + x)
 // + sqrt(1 + y)): accurate as B -> 0.  J = det F as in the reference.
+// LIMIT: only where spectral_as_accurate (a caller whose F may be of any strain).
 // ---------------------------------------------------------------------------
+template <bool LIMIT = false>
 __device__ __forceinline__ bool jelly_stress_spectral(const MpmScene &S, const float Ft[9], float Fo[9],
                                                       float tau[9]) {
     const float J = Ft[0] * (Ft[4] * Ft[8] - Ft[5] * Ft[7]) - Ft[1] * (Ft[3] * Ft[8] - Ft[5] * Ft[6]) +
@@ -643,7 +657,7 @@ __device__ __forceinline__ bool jelly_stress_spectral(const MpmScene &S, const f
     float B[6], ev[3];
     left_strain(Ft, B);
     sym_eig3(B, ev);
-    if (!(ev[2] > -0.99f)) return false;
+    if (!(LIMIT ? spectral_as_accurate(ev) : ev[2] > -0.99f)) return false;
     Newton3 N;
     newton3_setup(B, ev, N);
     const float r0 = sqrtf(1.0f + ev[0]), r1 = sqrtf(1.0f + ev[1]), r2 = sqrtf(1.0f + ev[2]);

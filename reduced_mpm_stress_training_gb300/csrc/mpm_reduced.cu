@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256) mark_kernel(const MpmScene *__restrict__ 
 // lam tr(E) I with E = log(F F^T) / 2, in Newton form on the closed-form
 // eigenvalues of B = F F^T - I (as sand_return_map_spectral, which also says
 // why it is the more accurate form near F = I).  False (SVD path) for inverted
-// or extremely compressed elements.
+// elements and where the strain makes the SVD the more accurate one.
 __device__ __forceinline__ bool stress_dp_spectral(const float F[9], float mu, float lam, float tau[9]) {
     const float J = F[0] * (F[4] * F[8] - F[5] * F[7]) - F[1] * (F[3] * F[8] - F[5] * F[6]) +
                     F[2] * (F[3] * F[7] - F[4] * F[6]);
@@ -126,7 +126,7 @@ __device__ __forceinline__ bool stress_dp_spectral(const float F[9], float mu, f
     float B[6], ev[3];
     left_strain(F, B);
     sym_eig3(B, ev);
-    if (!(ev[2] > -0.99f)) return false;
+    if (!spectral_as_accurate(ev)) return false;
     const float e0 = 0.5f * log1pf(ev[0]), e1 = 0.5f * log1pf(ev[1]), e2 = 0.5f * log1pf(ev[2]);
     const float q0 = 1.0f + ev[0], q1 = 1.0f + ev[1], q2 = 1.0f + ev[2];
     Newton3 N;
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kRedWarps * 32) reduced_p2g_kernel(const MpmSc
         stpair(st, i, 0, q0, make_float4(q1.x, q1.y, q1.z, F[8]));
         stpair(st, i, 4, make_float4(F[0], F[1], F[2], F[3]), make_float4(F[4], F[5], F[6], F[7]));
         const bool sand = S.material == MPM_SAND;
-        if (!(sand ? stress_dp_spectral(F, S.mu, S.lam, tau) : jelly_stress_spectral(S, F, Fo, tau))) {
+        if (!(sand ? stress_dp_spectral(F, S.mu, S.lam, tau) : jelly_stress_spectral<true>(S, F, Fo, tau))) {
             Svd d;
             svd3(F, d);
             if (sand) stress_dp(F, d, S.mu, S.lam, tau);
