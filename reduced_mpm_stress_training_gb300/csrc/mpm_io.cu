@@ -112,18 +112,28 @@ cudaError_t launch_slot_of_uid(const Ctx &cx) {
 
 // load_uvstress_from_tensor (mpm_solver_warp.py:253-266) in one pass: u, v
 // and stress of user particle `id` into its record (quads 2, 3, 5-7; the C
-// words sharing quads 3 and 5 are kept)
+// words sharing quads 3 and 5 are kept).  The first `blocks` blocks write u and v (pair 1),
+// the others the stress (pairs 2, 3): user order is often no order of the slots, and
+// blocks that run together then scatter into one or two of the five pair arrays, which
+// L2 holds longer than all three.
 __global__ void load_uvstress_kernel(PState st, int n, const int *__restrict__ inv, const float *__restrict__ u,
-                                     const float *__restrict__ v, const float *__restrict__ tau) {
+                                     const float *__restrict__ v, const float *__restrict__ tau, int blocks) {
     chain_wait();
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool second = (int)blockIdx.x >= blocks;
+    const int id = ((int)blockIdx.x - (second ? blocks : 0)) * blockDim.x + threadIdx.x;
     if (id >= n) return;
     const int i = inv[id];
-    const float4 q3 = ldrec(st, i, 3), q5 = ldrec(st, i, 5);
-    const float *pu = u + (int64_t)id * 3, *pv = v + (int64_t)id * 3, *pt = tau + (int64_t)id * 9;
-    stpair(st, i, 1, make_float4(pu[0], pu[1], pu[2], pv[0]), make_float4(pv[1], pv[2], q3.z, q3.w));
-    strec(st, i, 5, make_float4(q5.x, q5.y, q5.z, pt[0]));
-    stpair(st, i, 3, make_float4(pt[1], pt[2], pt[3], pt[4]), make_float4(pt[5], pt[6], pt[7], pt[8]));
+    if (!second) {
+        const float4 q3 = ldrec(st, i, 3);
+        const float *pu = u + (int64_t)id * 3, *pv = v + (int64_t)id * 3;
+        stpair(st, i, 1, make_float4(pu[0], pu[1], pu[2], pv[0]), make_float4(pv[1], pv[2], q3.z, q3.w));
+    } else {
+        const float *pt = tau + (int64_t)id * 9;
+        float4 q4, q5;
+        ldpair(st, i, 2, q4, q5);
+        stpair(st, i, 2, q4, make_float4(q5.x, q5.y, q5.z, pt[0]));
+        stpair(st, i, 3, make_float4(pt[1], pt[2], pt[3], pt[4]), make_float4(pt[5], pt[6], pt[7], pt[8]));
+    }
 }
 
 // export_uvFstress_from_warp (mpm_solver_warp.py:305-310) in one pass: u, v,
@@ -184,26 +194,39 @@ __global__ void __launch_bounds__(kExportWarps * 32) export_uvFstress_kernel(
 // consecutive floats.  out: x_initial (3, n) | q = u (3, n) | masses (1, n) |
 // f_tensor = F - I (9, n) | stress components 0,1,2,4,5,8 (6, n) | v (3, n) |
 // C (9, n).
-__global__ void export_frame_kernel(PState st, int n, const int *__restrict__ inv, float *__restrict__ out) {
+// Each fifth of the blocks reads one pair array: user order is often no order of the
+// slots, and one array at a time stays in L2 where five do not.
+__global__ void export_frame_kernel(PState st, int n, const int *__restrict__ inv, float *__restrict__ out,
+                                    int blocks) {
     chain_wait();
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
+    const int pair = (int)blockIdx.x / blocks;
+    const int id = ((int)blockIdx.x - pair * blocks) * blockDim.x + threadIdx.x;
     if (id >= n) return;
-    const int i = inv[id];
-    const float4 q0 = ldrec(st, i, 0), q1 = ldrec(st, i, 1), q2 = ldrec(st, i, 2), q3 = ldrec(st, i, 3),
-                 q4 = ldrec(st, i, 4), q5 = ldrec(st, i, 5), q6 = ldrec(st, i, 6), q7 = ldrec(st, i, 7),
-                 q8 = ldrec(st, i, 8), q9 = ldrec(st, i, 9);
+    float4 a, b;
+    ldpair(st, inv[id], pair, a, b);
     const int64_t N = n;
     float *o = out + id;
-    const float rows[34] = {
-        q0.x, q0.y, q0.z,                                                                    // x
-        q2.x, q2.y, q2.z,                                                                    // q
-        q0.w,                                                                                // masses
-        q8.x - 1.0f, q8.y, q8.z, q8.w, q9.x - 1.0f, q9.y, q9.z, q9.w, q1.w - 1.0f,           // f_tensor
-        q5.w, q6.x, q6.y, q6.w, q7.x, q7.w,                                                  // stress
-        q2.w, q3.x, q3.y,                                                                    // v
-        q3.z, q3.w, q4.x, q4.y, q4.z, q4.w, q5.x, q5.y, q5.z};                               // C
-#pragma unroll
-    for (int r = 0; r < 34; ++r) o[r * N] = rows[r];
+    auto row = [&](int r, float v) { o[r * N] = v; };
+    switch (pair) {  // rows: x 0-2, q 3-5, masses 6, f_tensor 7-15, stress 16-21, v 22-24, C 25-33
+        case 0:
+            row(0, a.x); row(1, a.y); row(2, a.z); row(6, a.w); row(15, b.w - 1.0f);
+            break;
+        case 1:
+            row(3, a.x); row(4, a.y); row(5, a.z); row(22, a.w); row(23, b.x); row(24, b.y);
+            row(25, b.z); row(26, b.w);
+            break;
+        case 2:
+            row(27, a.x); row(28, a.y); row(29, a.z); row(30, a.w); row(31, b.x); row(32, b.y); row(33, b.z);
+            row(16, b.w);
+            break;
+        case 3:
+            row(17, a.x); row(18, a.y); row(19, a.w); row(20, b.x); row(21, b.w);
+            break;
+        default:
+            row(7, a.x - 1.0f); row(8, a.y); row(9, a.z); row(10, a.w); row(11, b.x - 1.0f); row(12, b.y);
+            row(13, b.z); row(14, b.w);
+            break;
+    }
 }
 
 // dense (n,n,n) grid_m / grid_v_in from the accumulator (valid after p2g)
@@ -296,8 +319,9 @@ cudaError_t launch_export(const Ctx &cx, int field, float *dst) {
 cudaError_t launch_load_uvstress(const Ctx &cx, const float *u, const float *v, const float *tau) {
     if (cx.n == 0) return cudaSuccess;
     launch_chained(slot_of_uid_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid);
-    launch_chained(load_uvstress_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid, u,
-                   v, tau);
+    const int blocks = (int)blocks_for(cx.n, 256);
+    launch_chained(load_uvstress_kernel, 2 * (int64_t)blocks, 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid, u, v,
+                   tau, blocks);
     return cudaGetLastError();
 }
 
@@ -312,7 +336,9 @@ cudaError_t launch_export_uvFstress(const Ctx &cx, float *u, float *v, float *fd
 cudaError_t launch_export_frame(const Ctx &cx, float *out) {
     if (cx.n == 0) return cudaSuccess;
     launch_chained(slot_of_uid_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid);
-    launch_chained(export_frame_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid, out);
+    const int blocks = (int)blocks_for(cx.n, 256);
+    launch_chained(export_frame_kernel, 5 * (int64_t)blocks, 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid, out,
+                   blocks);
     return cudaGetLastError();
 }
 
