@@ -401,13 +401,16 @@ __device__ void stage(const MpmStressDecoder &d, const float *label, Smem<P> &s)
 
 // the 128 threads of pipeline `pipe`: a barrier, and one whose outcome is the
 // AND of every thread's flag (named barriers 1 and 2; 0 is __syncthreads)
-// (barrier ids are immediates, so the kernel reserves three barriers, not sixteen)
+// (barrier ids are immediates, so the kernel reserves three barriers, not sixteen;
+// bar is warp-wide (.aligned): the lanes are brought together first)
 __device__ __forceinline__ void pipe_sync(int pipe) {
+    __syncwarp();
     if (pipe == 0) asm volatile("bar.sync 1, 128;\n" ::: "memory");
     else asm volatile("bar.sync 2, 128;\n" ::: "memory");
 }
 __device__ __forceinline__ bool pipe_and(int pipe, bool v) {
     uint32_t r;
+    __syncwarp();
     if (pipe == 0)
         asm volatile(
             "{\n.reg .pred p, q;\nsetp.ne.u32 q, %1, 0;\nbar.red.and.pred p, 1, 128, q;\nselp.u32 %0, 1, 0, p;\n}\n"
@@ -445,6 +448,7 @@ __global__ void __launch_bounds__(P * dtc::kRows, P == 2 ? 3 : 4) decoder_stress
     }
     if (warp == 0) {
         const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&s.tmem_base);
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(dst),
                      "r"(kTmemCols * P)
                      : "memory");
@@ -560,10 +564,12 @@ __global__ void __launch_bounds__(P * dtc::kRows, P == 2 ? 3 : 4) decoder_stress
     mlptc::tc_before_sync();
     __syncthreads();
     mlptc::tc_after_sync();
-    if (warp == 0)
+    if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(s.tmem_base),
                      "r"(kTmemCols * P)
                      : "memory");
+    }
 }
 
 int64_t decoder_param_floats(const MpmStressDecoder &d) {

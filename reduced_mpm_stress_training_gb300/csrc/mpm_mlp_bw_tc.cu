@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) mlp_backward_tc_kernel(const __
     }
     if (warp == 0) {
         const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&s.tmem_base);
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(dst),
                      "r"(kBwCols)
                      : "memory");
@@ -379,9 +380,11 @@ __global__ void __launch_bounds__(kBwThreads, 1) mlp_backward_tc_kernel(const __
     tc_before_sync();
     __syncthreads();
     tc_after_sync();
-    if (warp == 0)
+    if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tbase), "r"(kBwCols)
                      : "memory");
+    }
 }
 
 }  // namespace mlpbw

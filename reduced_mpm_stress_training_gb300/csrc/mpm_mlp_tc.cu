@@ -92,7 +92,9 @@ __device__ __forceinline__ void stage_forward(FwSmem &s, const __nv_bfloat16 *w,
 }
 
 // barrier over the 256 threads of a pipeline (ids 1 .. kPipes; immediates, so that the
-// kernel reserves no more barriers than it uses)
+// kernel reserves no more barriers than it uses).  bar.sync is warp-wide (.aligned), as
+// tcgen05.ld is: the kernel brings a warp's lanes together where they may have parted (the
+// rows past n, the poll loop) and not before each of these (1M rows 183 us, 187 so).
 __device__ __forceinline__ void pipe_barrier(int pipe) {
     static_assert(kPipes == 3 && kThreads == 256, "barrier ids and counts");
     if (pipe == 0) asm volatile("bar.sync 1, 256;\n" ::: "memory");
@@ -161,6 +163,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) mlp_forward_tc_kernel(const __n
     }
     if (threadIdx.x < 32) {
         const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&s.tmem_base);
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(dst), "r"(kFwCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
@@ -198,6 +201,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) mlp_forward_tc_kernel(const __n
             for (int k = 0; k < IN; ++k) xv[k] = 0.0f;
             if (next < io.n) load_x(io, next, xv);
         }
+        __syncwarp();
 #pragma unroll 1
         for (int layer = 0; layer < 4; ++layer) {
             fence_async_smem();
@@ -222,6 +226,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) mlp_forward_tc_kernel(const __n
                 mma_commit(mbar);
             }
             if (!mbar_wait(mbar, phase)) *fail = 1;
+            __syncwarp();
             phase ^= 1u;
             tc_after_sync();
             if (layer == 3) break;
@@ -230,13 +235,14 @@ __global__ void __launch_bounds__(kFwThreads, 1) mlp_forward_tc_kernel(const __n
 #pragma unroll 1
             for (int c0 = half * (H / 2); c0 < (half + 1) * (H / 2); c0 += 32) {
                 float acc[32];
-                tmem_ld32(tlane + (uint32_t)c0, acc);
+                tmem_ld32<true>(tlane + (uint32_t)c0, acc);
                 activate_chunk(sh, acc, s.bias + layer * H, row, c0, zrow);
+                if (io.z) __syncwarp();  // rows past n store no Z
             }
         }
         if (!ok) break;
         float acc[32];
-        tmem_ld32(tlane, acc);
+        tmem_ld32<true>(tlane, acc);
 #pragma unroll
         for (int c = 0; c < OUT; ++c) acc[c] += s.b4[c];
         if (lead && valid) {
@@ -284,9 +290,11 @@ __global__ void __launch_bounds__(kFwThreads, 1) mlp_forward_tc_kernel(const __n
         atomicAdd(io.loss, sum);
     }
     __syncthreads();
-    if (threadIdx.x < 32)
+    if (threadIdx.x < 32) {
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(s.tmem_base), "r"(kFwCols)
                      : "memory");
+    }
 }
 
 }  // namespace mlptc

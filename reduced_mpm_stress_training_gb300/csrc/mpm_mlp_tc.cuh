@@ -79,8 +79,13 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *mbar, uint32_t par
     return false;
 }
 
+// 32 accumulator columns of this thread's row.  The instructions are warp-wide (.aligned):
+// the lanes may come from a poll loop that they left one by one, so they are brought
+// together first, unless the caller has done so (TOGETHER).
+template <bool TOGETHER = false>
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float v[32]) {
     uint32_t r[32];
+    if (!TOGETHER) __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
         "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
@@ -150,6 +155,7 @@ __device__ __forceinline__ uint32_t tc_setup(TcSmem &s, const __nv_bfloat16 *w, 
     }
     if (warp == 0) {
         const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&s.tmem_base);
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(dst),
                      "r"(kTmemCols)
                      : "memory");
@@ -170,6 +176,7 @@ __device__ __forceinline__ void tc_teardown(TcSmem &s, uint32_t tbase, bool ok, 
     tc_after_sync();
     if ((threadIdx.x >> 5) == 0) {
         if (!ok) mbar_wait(&s.mbar, phase ^ 1u);
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tbase), "r"(kTmemCols)
                      : "memory");
     }
