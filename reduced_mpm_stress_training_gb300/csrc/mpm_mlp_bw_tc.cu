@@ -221,6 +221,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) mlp_backward_tc_kernel(const __
         tc_after_sync();
     };
     auto failed = [&]() { return *reinterpret_cast<volatile int *>(&s.fail) != 0; };
+    bool stopped = false;     // a wait ran out (uniform: read behind a barrier)
     uint32_t zl[16], zp[16];  // Z of this phase's data gradient, Z of its activations
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int64_t row0 = tile * kRows, grow = row0 + row;
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) mlp_backward_tc_kernel(const __
         cp_commit();
         cp_wait<1>();     // Z3
         __syncthreads();  // every thread's part of it
-        if (failed()) break;
+        if ((stopped = failed())) break;
         activate(s.h[a], row, c0, zl);
         if (quarter == 0) {
             *reinterpret_cast<uint4 *>(s.dz4 + core_off<2>(row, 0)) = d0;
@@ -275,7 +276,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) mlp_backward_tc_kernel(const __
         cp_wait<0>();  // Z2
         data_gradient(s.dz[0], tlane + C_DH, row, c0, zl);
         __syncthreads();
-        if (failed()) break;
+        if ((stopped = failed())) break;
         activate(s.h[a ^ 1], row, c0, zp);
         bw_sync();
         if (tid == 0) {
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) mlp_backward_tc_kernel(const __
         data_gradient(s.dz[1], tlane + C_DH, row, c0, zp);
         cp_wait<0>();
         __syncthreads();
-        if (failed()) break;
+        if ((stopped = failed())) break;
         activate(s.h[a], row, c0, zl);
         bw_sync();
         if (tid == 0) {
@@ -320,7 +321,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) mlp_backward_tc_kernel(const __
         cp_commit();
         data_gradient(s.dz[0], tlane + C_DH, row, c0, zl);
         bw_sync();
-        if (failed()) break;
+        if ((stopped = failed())) break;
         if (tid == 0) {
 #pragma unroll 1
             for (int ks = 0; ks < 8; ++ks)
@@ -332,7 +333,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) mlp_backward_tc_kernel(const __
         a ^= 1;
     }
     cp_wait<0>();
-    if (!first || failed()) wait_mma();  // (after a timeout: the bounded grace wait)
+    if (!stopped && !first) wait_mma();  // the last tile's weight gradients
     tc_before_sync();
     __syncthreads();
     tc_after_sync();
@@ -376,7 +377,14 @@ __global__ void __launch_bounds__(kBwThreads, 1) mlp_backward_tc_kernel(const __
             }
         }
     }
-    if (!ok && tid == 0) atomicOr(err, 1);
+    if (!ok && tid == 0) {
+        atomicOr(err, 1);
+        // before the tensor memory is released, a bounded grace wait for the MMAs in flight:
+        // for the commit whose wait ran out, and for those issued since
+        mma_commit(&s.mbar);
+        mbar_wait(&s.mbar, phase ^ 1u);
+        mbar_wait(&s.mbar, phase);
+    }
     tc_before_sync();
     __syncthreads();
     tc_after_sync();
