@@ -124,8 +124,8 @@ typedef struct MpmPlan {
 } MpmPlan; /* 56 bytes */
 
 /* Caller-owned device buffers plus the host-side control the library keeps
- * between calls.  All pointers are device pointers (256-byte aligned; calls
- * refuse state buffers that are not at least 32-byte aligned). */
+ * between calls.  All pointers are device pointers (256-byte aligned; state
+ * buffers of 16-byte alignment are served, more slowly, and less is refused). */
 typedef struct MpmBuffers {
     void *state[2];   /* two particle-state buffers, plan.state_bytes each      */
     void *workspace;  /* plan.workspace_bytes                                  */

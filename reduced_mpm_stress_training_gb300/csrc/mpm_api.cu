@@ -108,6 +108,7 @@ mpm::PState state_view(void *base, int64_t stride) {
     s.stride = stride;
     s.q = reinterpret_cast<float4 *>(p);
     s.key = reinterpret_cast<int *>(p + stride * mpm::kRecWords * 4);
+    s.wide = (reinterpret_cast<uintptr_t>(base) & 31) == 0;
     return s;
 }
 
@@ -151,11 +152,11 @@ mpm::Ctx make_ctx(const MpmBuffers *b, void *stream, int which) {
     return cx;
 }
 
-// (the state's records move in 32-byte accesses)
+// (the state's records move in accesses of at least 16 bytes)
 bool buffers_ok(const MpmBuffers *b) {
-    return b && b->state[0] && b->state[1] &&
-           !((reinterpret_cast<uintptr_t>(b->state[0]) | reinterpret_cast<uintptr_t>(b->state[1])) & 31) && b->workspace && b->scenes && b->status &&
-           b->plan.n_scenes >= 1 && (b->cur == 0 || b->cur == 1);
+    if (!b || !b->state[0] || !b->state[1] || !b->workspace || !b->scenes || !b->status) return false;
+    if ((reinterpret_cast<uintptr_t>(b->state[0]) | reinterpret_cast<uintptr_t>(b->state[1])) & 15) return false;
+    return b->plan.n_scenes >= 1 && (b->cur == 0 || b->cur == 1);
 }
 
 }  // namespace

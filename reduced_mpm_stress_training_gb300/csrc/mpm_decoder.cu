@@ -208,18 +208,19 @@ __global__ void __launch_bounds__(kDecThreads) decoder_rows_kernel(MpmStressDeco
 }
 
 // the symmetric stress of the six components into the record, whole pairs (sectors) at a time
+template <bool NARROW>
 __device__ __forceinline__ void store_stress(const PState &st, int i, const float q[6]) {
     float4 q4, q5;
-    ldpair(st, i, 2, q4, q5);
-    stpair(st, i, 2, q4, make_float4(q5.x, q5.y, q5.z, q[0]));
-    stpair(st, i, 3, make_float4(q[1], q[2], q[1], q[3]), make_float4(q[4], q[2], q[4], q[5]));
+    ldpair<NARROW>(st, i, 2, q4, q5);
+    stpair<NARROW>(st, i, 2, q4, make_float4(q5.x, q5.y, q5.z, q[0]));
+    stpair<NARROW>(st, i, 3, make_float4(q[1], q[2], q[1], q[3]), make_float4(q[4], q[2], q[4], q[5]));
 }
 
 // The decoder as the stress source of a substep: label (label_dim floats, the
 // frame's latent), each particle's x_initial from its record and mu row
 // (mu_dim floats, user order) by uid; writes the symmetric stress
 // [q0 q1 q2; q1 q3 q4; q2 q4 q5] into the record (mpm_solver_warp.py:383 order).
-template <int HP>
+template <int HP, bool NARROW>
 __global__ void __launch_bounds__(kDecThreads) decoder_stress_kernel(MpmStressDecoder d, PState st,
                                                                      const float *__restrict__ label,
                                                                      const float *__restrict__ mu, int n) {
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(kDecThreads) decoder_stress_kernel(MpmStressDe
         for (int j = 0; j < HP; ++j) h[j] = dec_act(h[j], siren, d.omega_0);
         float q[6];
         dec_tail<HP>(sm, L, h, siren, d.omega_0, q);
-        store_stress(st, i, q);
+        store_stress<NARROW>(st, i, q);
     }
 }
 
@@ -428,7 +429,7 @@ __device__ __forceinline__ bool pipe_and(int pipe, bool v) {
 
 }  // namespace dtc
 
-template <int P>
+template <int P, bool NARROW>
 __global__ void __launch_bounds__(P * dtc::kRows, P == 2 ? 3 : 4) decoder_stress_tc_kernel(MpmStressDecoder d, PState st,
                                                                           const float *__restrict__ label,
                                                                           const float *__restrict__ mu, int n,
@@ -552,7 +553,7 @@ __global__ void __launch_bounds__(P * dtc::kRows, P == 2 ? 3 : 4) decoder_stress
             q[c] = __fadd_rn(s.qm[c], __fmul_rn(acc.x + acc.y, s.qs[c]));
         }
         if (live) {
-            store_stress(st, i, q);
+            store_stress<NARROW>(st, i, q);
         }
     }
     if (!ok && row == 0) {
@@ -633,18 +634,21 @@ cudaError_t launch_decoder_stress(const Ctx &cx, const MpmStressDecoder &d, cons
         if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
         const int bytes = (int)sizeof(dtc::Smem<P>);
         if (!attr[dev]) {
-            e = cudaFuncSetAttribute(decoder_stress_tc_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-            if (e != cudaSuccess) return e;
+            for (auto kernel : {decoder_stress_tc_kernel<P, false>, decoder_stress_tc_kernel<P, true>}) {
+                e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+                if (e != cudaSuccess) return e;
+            }
             attr[dev] = true;
         }
         const int tiles = (cx.n + dtc::kRows - 1) / dtc::kRows;
         const int groups = (tiles + P - 1) / P;
         const int tgrid = groups < cx.num_sms * per_sm ? groups : cx.num_sms * per_sm;
-        launch_chained(decoder_stress_tc_kernel<P>, tgrid, P * dtc::kRows, bytes, cx.stream, d, cx.st, label, mu, cx.n,
-                                                                                 cx.status);
+        launch_chained(cx.st.wide ? decoder_stress_tc_kernel<P, false> : decoder_stress_tc_kernel<P, true>, tgrid,
+                       P * dtc::kRows, bytes, cx.stream, d, cx.st, label, mu, cx.n, cx.status);
     } else {
-        if ((e = dec_prepare(decoder_stress_kernel<64>, 3)) != cudaSuccess) return e;
-        launch_chained(decoder_stress_kernel<64>, grid, kDecThreads, smem, cx.stream, d, cx.st, label, mu, cx.n);
+        const auto kernel = cx.st.wide ? decoder_stress_kernel<64, false> : decoder_stress_kernel<64, true>;
+        if ((e = dec_prepare(kernel, cx.st.wide ? 2 : 3)) != cudaSuccess) return e;
+        launch_chained(kernel, grid, kDecThreads, smem, cx.stream, d, cx.st, label, mu, cx.n);
     }
     return cudaGetLastError();
 }

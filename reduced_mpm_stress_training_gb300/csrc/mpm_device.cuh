@@ -47,6 +47,7 @@ struct PState {
     float4 *q;    // pair p of slot s: q[(p * stride + s) * 2] and the quad after it
     int *key;     // cell key (block * 64 + cell in block) of each slot for the coming sort
     int64_t stride;
+    bool wide;    // the buffer is 32-byte aligned: a pair moves in one access
 };
 
 // address of record quad q (0..9) of a slot
@@ -55,16 +56,30 @@ __device__ __forceinline__ float4 *recq(const PState &st, int slot, int q) {
 }
 __device__ __forceinline__ float4 ldrec(const PState &st, int slot, int q) { return *recq(st, slot, q); }
 __device__ __forceinline__ void strec(const PState &st, int slot, int q, float4 v) { *recq(st, slot, q) = v; }
-// both quads of a pair in one 32-byte access (the state buffers are 256-byte aligned)
+// both quads of a pair: in one 32-byte access, or (NARROW: the caller's buffer allows no
+// more) in two of 16 bytes.  The launch chooses: where a kernel asked, its loads waited
+// for one another (export of 8M particles 389 -> 623 us).
+template <bool NARROW>
 __device__ __forceinline__ void ldpair(const PState &st, int slot, int p, float4 &a, float4 &b) {
-    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-                 : "l"(recq(st, slot, 2 * p)));
+    if (!NARROW) {
+        asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                     : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                     : "l"(recq(st, slot, 2 * p)));
+    } else {
+        a = ldrec(st, slot, 2 * p);
+        b = ldrec(st, slot, 2 * p + 1);
+    }
 }
+template <bool NARROW>
 __device__ __forceinline__ void stpair(const PState &st, int slot, int p, const float4 &a, const float4 &b) {
-    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(recq(st, slot, 2 * p)), "f"(a.x),
-                 "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
-                 : "memory");
+    if (!NARROW) {
+        asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(recq(st, slot, 2 * p)), "f"(a.x),
+                     "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                     : "memory");
+    } else {
+        strec(st, slot, 2 * p, a);
+        strec(st, slot, 2 * p + 1, b);
+    }
 }
 // record word w (0..39) of a slot
 __device__ __forceinline__ float &recword(const PState &st, int slot, int w) {

@@ -116,6 +116,7 @@ cudaError_t launch_slot_of_uid(const Ctx &cx) {
 // the others the stress (pairs 2, 3): user order is often no order of the slots, and
 // blocks that run together then scatter into one or two of the five pair arrays, which
 // L2 holds longer than all three.
+template <bool NARROW>
 __global__ void load_uvstress_kernel(PState st, int n, const int *__restrict__ inv, const float *__restrict__ u,
                                      const float *__restrict__ v, const float *__restrict__ tau, int blocks) {
     chain_wait();
@@ -126,13 +127,13 @@ __global__ void load_uvstress_kernel(PState st, int n, const int *__restrict__ i
     if (!second) {
         const float4 q3 = ldrec(st, i, 3);
         const float *pu = u + (int64_t)id * 3, *pv = v + (int64_t)id * 3;
-        stpair(st, i, 1, make_float4(pu[0], pu[1], pu[2], pv[0]), make_float4(pv[1], pv[2], q3.z, q3.w));
+        stpair<NARROW>(st, i, 1, make_float4(pu[0], pu[1], pu[2], pv[0]), make_float4(pv[1], pv[2], q3.z, q3.w));
     } else {
         const float *pt = tau + (int64_t)id * 9;
         float4 q4, q5;
-        ldpair(st, i, 2, q4, q5);
-        stpair(st, i, 2, q4, make_float4(q5.x, q5.y, q5.z, pt[0]));
-        stpair(st, i, 3, make_float4(pt[1], pt[2], pt[3], pt[4]), make_float4(pt[5], pt[6], pt[7], pt[8]));
+        ldpair<NARROW>(st, i, 2, q4, q5);
+        stpair<NARROW>(st, i, 2, q4, make_float4(q5.x, q5.y, q5.z, pt[0]));
+        stpair<NARROW>(st, i, 3, make_float4(pt[1], pt[2], pt[3], pt[4]), make_float4(pt[5], pt[6], pt[7], pt[8]));
     }
 }
 
@@ -142,6 +143,7 @@ __global__ void load_uvstress_kernel(PState st, int n, const int *__restrict__ i
 // rows of 12 and 36 bytes written by one lane each touch 3 and 9 lines per
 // store instruction.  Measured on the 1M column: 95 -> 55 us.
 constexpr int kExportWarps = 4;
+template <bool NARROW>
 __global__ void __launch_bounds__(kExportWarps * 32) export_uvFstress_kernel(
     PState st, int n, const int *__restrict__ inv, float *__restrict__ u, float *__restrict__ v,
     float *__restrict__ fd, float *__restrict__ tau) {
@@ -153,11 +155,11 @@ __global__ void __launch_bounds__(kExportWarps * 32) export_uvFstress_kernel(
     if (id < n) {
         const int i = inv[id];
         float4 q0, q1, q2, q3, q6, q7, q8, q9;
-        ldpair(st, i, 0, q0, q1);
-        ldpair(st, i, 1, q2, q3);
+        ldpair<NARROW>(st, i, 0, q0, q1);
+        ldpair<NARROW>(st, i, 1, q2, q3);
         const float4 q5 = ldrec(st, i, 5);
-        ldpair(st, i, 3, q6, q7);
-        ldpair(st, i, 4, q8, q9);
+        ldpair<NARROW>(st, i, 3, q6, q7);
+        ldpair<NARROW>(st, i, 4, q8, q9);
         float *pu = mine + lane * 3, *pv = mine + 96 + lane * 3, *pf = mine + 192 + lane * 9,
               *pt = mine + 480 + lane * 9;
         pu[0] = q2.x; pu[1] = q2.y; pu[2] = q2.z;
@@ -196,6 +198,7 @@ __global__ void __launch_bounds__(kExportWarps * 32) export_uvFstress_kernel(
 // C (9, n).
 // Each fifth of the blocks reads one pair array: user order is often no order of the
 // slots, and one array at a time stays in L2 where five do not.
+template <bool NARROW>
 __global__ void export_frame_kernel(PState st, int n, const int *__restrict__ inv, float *__restrict__ out,
                                     int blocks) {
     chain_wait();
@@ -203,7 +206,7 @@ __global__ void export_frame_kernel(PState st, int n, const int *__restrict__ in
     const int id = ((int)blockIdx.x - pair * blocks) * blockDim.x + threadIdx.x;
     if (id >= n) return;
     float4 a, b;
-    ldpair(st, inv[id], pair, a, b);
+    ldpair<NARROW>(st, inv[id], pair, a, b);
     const int64_t N = n;
     float *o = out + id;
     auto row = [&](int r, float v) { o[r * N] = v; };
@@ -320,16 +323,17 @@ cudaError_t launch_load_uvstress(const Ctx &cx, const float *u, const float *v, 
     if (cx.n == 0) return cudaSuccess;
     launch_chained(slot_of_uid_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid);
     const int blocks = (int)blocks_for(cx.n, 256);
-    launch_chained(load_uvstress_kernel, 2 * (int64_t)blocks, 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid, u, v,
-                   tau, blocks);
+    launch_chained(cx.st.wide ? load_uvstress_kernel<false> : load_uvstress_kernel<true>, 2 * (int64_t)blocks, 256, 0,
+                   cx.stream, cx.st, cx.n, cx.ws.slot_of_uid, u, v, tau, blocks);
     return cudaGetLastError();
 }
 
 cudaError_t launch_export_uvFstress(const Ctx &cx, float *u, float *v, float *fd, float *tau) {
     if (cx.n == 0) return cudaSuccess;
     launch_chained(slot_of_uid_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid);
-    launch_chained(export_uvFstress_kernel, blocks_for(cx.n, kExportWarps * 32), kExportWarps * 32, 0, cx.stream,
-        cx.st, cx.n, cx.ws.slot_of_uid, u, v, fd, tau);
+    launch_chained(cx.st.wide ? export_uvFstress_kernel<false> : export_uvFstress_kernel<true>,
+                   blocks_for(cx.n, kExportWarps * 32), kExportWarps * 32, 0, cx.stream, cx.st, cx.n,
+                   cx.ws.slot_of_uid, u, v, fd, tau);
     return cudaGetLastError();
 }
 
@@ -337,8 +341,8 @@ cudaError_t launch_export_frame(const Ctx &cx, float *out) {
     if (cx.n == 0) return cudaSuccess;
     launch_chained(slot_of_uid_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid);
     const int blocks = (int)blocks_for(cx.n, 256);
-    launch_chained(export_frame_kernel, 5 * (int64_t)blocks, 256, 0, cx.stream, cx.st, cx.n, cx.ws.slot_of_uid, out,
-                   blocks);
+    launch_chained(cx.st.wide ? export_frame_kernel<false> : export_frame_kernel<true>, 5 * (int64_t)blocks, 256, 0,
+                   cx.stream, cx.st, cx.n, cx.ws.slot_of_uid, out, blocks);
     return cudaGetLastError();
 }
 

@@ -69,7 +69,7 @@ void *noalloc_workspace(int *err) {
 extern "C" int mpm_p2g2p_noalloc(MpmBuffers *b, float time, float dt, void *stream) {
     if (!b || !b->state[0] || !b->state[1] || !b->scenes || !b->status) return MPM_ERR_ARG;
     // as every entry point (checked here before the array is cleared)
-    if ((reinterpret_cast<uintptr_t>(b->state[0]) | reinterpret_cast<uintptr_t>(b->state[1])) & 31) return MPM_ERR_ARG;
+    if ((reinterpret_cast<uintptr_t>(b->state[0]) | reinterpret_cast<uintptr_t>(b->state[1])) & 15) return MPM_ERR_ARG;
     const int64_t need = mpm::substep_workspace_bytes(b->plan);
     if (need < 0 || (size_t)need > kNoAllocWorkspaceBytes) return MPM_ERR_SIZE;
     int err = MPM_OK;

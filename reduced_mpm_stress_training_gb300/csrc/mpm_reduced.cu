@@ -157,6 +157,7 @@ __device__ __forceinline__ bool stress_dp_spectral(const float F[9], float mu, f
 // an SVD per stress and segmented shuffles over the runs as they lie, 126 us.
 constexpr int kRedWarps = 4;
 constexpr int kRedPay = 5;  // float4 of a particle's scatter data
+template <bool NARROW>
 __global__ void __launch_bounds__(kRedWarps * 32) reduced_p2g_kernel(const MpmScene *__restrict__ scenes, PState st,
                                                                      MpmReducedGrid g, int n, float dt,
                                                                      int *status) {
@@ -173,8 +174,8 @@ __global__ void __launch_bounds__(kRedWarps * 32) reduced_p2g_kernel(const MpmSc
     int base[3] = {0, 0, 0};
     bool act = false;
     if (i < n) {
-        ldpair(st, i, 0, q0, q1);
-        ldpair(st, i, 1, q2, q3);
+        ldpair<NARROW>(st, i, 0, q0, q1);
+        ldpair<NARROW>(st, i, 1, q2, q3);
         const float gp[3] = {grid_coord(q0.x, q2.x, inv_dx), grid_coord(q0.y, q2.y, inv_dx),
                              grid_coord(q0.z, q2.z, inv_dx)};
         bool cell_in = true, stencil_in = true;
@@ -211,8 +212,8 @@ __global__ void __launch_bounds__(kRedWarps * 32) reduced_p2g_kernel(const MpmSc
         float F[9], tau[9], Fo[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) F[k] = __fadd_rn(fd[k], (k % 4 == 0) ? 1.0f : 0.0f);  // F_disp + I (:364)
-        stpair(st, i, 0, q0, make_float4(q1.x, q1.y, q1.z, F[8]));
-        stpair(st, i, 4, make_float4(F[0], F[1], F[2], F[3]), make_float4(F[4], F[5], F[6], F[7]));
+        stpair<NARROW>(st, i, 0, q0, make_float4(q1.x, q1.y, q1.z, F[8]));
+        stpair<NARROW>(st, i, 4, make_float4(F[0], F[1], F[2], F[3]), make_float4(F[4], F[5], F[6], F[7]));
         const bool sand = S.material == MPM_SAND;
         if (!(sand ? stress_dp_spectral(F, S.mu, S.lam, tau) : jelly_stress_spectral<true>(S, F, Fo, tau))) {
             Svd d;
@@ -439,8 +440,9 @@ cudaError_t launch_p2g2p_reduced(const Ctx &cx, const MpmReducedGrid &g, float t
         if (g.n_samples > 0)
             launch_chained(mark_kernel<2>, (unsigned)((g.n_samples + 7) / 8), 256, 0, cx.stream, cx.scenes, cx.st,
                            cx.ws.slot_of_uid, g, g.neighboring_cells, cx.n, cx.status);
-        launch_chained(reduced_p2g_kernel, (cx.n + kRedWarps * 32 - 1) / (kRedWarps * 32), kRedWarps * 32, 0,
-                       cx.stream, cx.scenes, cx.st, g, cx.n, dt, cx.status);
+        launch_chained(cx.st.wide ? reduced_p2g_kernel<false> : reduced_p2g_kernel<true>,
+                       (cx.n + kRedWarps * 32 - 1) / (kRedWarps * 32), kRedWarps * 32, 0, cx.stream, cx.scenes, cx.st, g,
+                       cx.n, dt, cx.status);
     }
     const int64_t want = (nn + 255) / 256;
     const int blocks = (int)(want < (int64_t)cx.num_sms * 16 ? want : (int64_t)cx.num_sms * 16);

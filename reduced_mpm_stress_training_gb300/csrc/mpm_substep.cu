@@ -160,6 +160,8 @@ __device__ __forceinline__ void p2g_flush(float4 *mytile, int cell, unsigned gma
     }
 }
 
+// NARROW: a state buffer of 16-byte alignment (see ldpair)
+template <bool NARROW>
 __global__ void __launch_bounds__(kP2GWarps * 32, 6) p2g_kernel(const MpmScene *__restrict__ scenes,
                                                                 int n_scenes, PState st, Ws ws, float dt,
                                                                 int *status) {
@@ -212,7 +214,7 @@ __global__ void __launch_bounds__(kP2GWarps * 32, 6) p2g_kernel(const MpmScene *
                 if (ok) {
                     float4 q[kP2GQuads];
 #pragma unroll
-                    for (int k = 0; k < kP2GQuads; k += 2) ldpair(st, slot, k / 2, q[k], q[k + 1]);
+                    for (int k = 0; k < kP2GQuads; k += 2) ldpair<NARROW>(st, slot, k / 2, q[k], q[k + 1]);
                     ok = p2g_load(S, q, bx, by, bz, dt, o) && (__float_as_int(o[1].w) >> 4) == warp;
                 }
                 if (!ok) {  // contributes zeros
@@ -456,12 +458,13 @@ __device__ __forceinline__ int g2p_slot(const Ws &ws, const int4 &ch) {
 
 // DEFER: leave the return map and stress to a later pass (the surrogate stress
 // stage): F_trial is stored as F and the stress words are zeroed.
-// FAST: the form that mpm_p2g2p runs, with five 128-thread CTAs per SM (96
-// registers) instead of four and less integer work.  The mpm_g2p stage and the
+// NARROW: `out` is a buffer of 16-byte alignment (see ldpair).
+// FAST: the form that mpm_p2g2p runs (on buffers that take 32-byte accesses), with five
+// 128-thread CTAs per SM (96 registers) instead of four and less integer work.  The mpm_g2p stage and the
 // ordered mode run the other form: ptxas fuses multiplies and adds differently
 // under another register budget, and they promise float32 results that stay
 // the same bit for bit (see mpm_ordered.cu).
-template <int CH, bool DEFER, bool FAST>
+template <int CH, bool DEFER, bool FAST, bool NARROW>
 __global__ void __launch_bounds__(CH, FAST ? 640 / CH : 0) g2p_kernel(const MpmScene *__restrict__ scenes, PState st,
                                                  PState out, Ws ws, float dt, int *status) {
     chain_wait();
@@ -649,14 +652,14 @@ __global__ void __launch_bounds__(CH, FAST ? 640 / CH : 0) g2p_kernel(const MpmS
 #pragma unroll
                 for (int k = 0; k < 9; ++k) chk += fabsf(Fo[k]) + fabsf(tau[k]);
                 if (!(S.material == MPM_METAL && S.hardening == 1)) yld = q1.z;
-                stpair(out, pos, 0, q0, make_float4(q1.x, q1.y, yld, Fo[8]));
-                stpair(out, pos, 1, make_float4(un[0], un[1], un[2], nv[0]),
+                stpair<NARROW>(out, pos, 0, q0, make_float4(q1.x, q1.y, yld, Fo[8]));
+                stpair<NARROW>(out, pos, 1, make_float4(un[0], un[1], un[2], nv[0]),
                        make_float4(nv[1], nv[2], nC[0], nC[1]));
-                stpair(out, pos, 2, make_float4(nC[2], nC[3], nC[4], nC[5]),
+                stpair<NARROW>(out, pos, 2, make_float4(nC[2], nC[3], nC[4], nC[5]),
                        make_float4(nC[6], nC[7], nC[8], tau[0]));
-                stpair(out, pos, 3, make_float4(tau[1], tau[2], tau[3], tau[4]),
+                stpair<NARROW>(out, pos, 3, make_float4(tau[1], tau[2], tau[3], tau[4]),
                        make_float4(tau[5], tau[6], tau[7], tau[8]));
-                stpair(out, pos, 4, make_float4(Fo[0], Fo[1], Fo[2], Fo[3]),
+                stpair<NARROW>(out, pos, 4, make_float4(Fo[0], Fo[1], Fo[2], Fo[3]),
                        make_float4(Fo[4], Fo[5], Fo[6], Fo[7]));
                 int flags = 0;
                 const float vmax = S.dx / dt;
@@ -693,7 +696,7 @@ static int persistent_grid(const Ctx &cx, int per_sm) {
 // spread over the whole list instead of sweeping it as one band, and the L2
 // reuse with P2G (the chunk list walked from its end) would fall: 200.2 ->
 // 198.8 us per substep on the 1M column against twice the resident count.
-template <int CH, bool DEFER, bool FAST>
+template <int CH, bool DEFER, bool FAST, bool NARROW>
 static cudaError_t g2p_t(const Ctx &cx, float dt) {
     // more than the 48 KB of static shared memory: opt in once per instance and device
     static int resident[64] = {0};
@@ -703,15 +706,15 @@ static cudaError_t g2p_t(const Ctx &cx, float dt) {
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (resident[dev] == 0) {
-        e = cudaFuncSetAttribute(g2p_kernel<CH, DEFER, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        e = cudaFuncSetAttribute(g2p_kernel<CH, DEFER, FAST, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return e;
         int nb = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, g2p_kernel<CH, DEFER, FAST>, CH, bytes);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, g2p_kernel<CH, DEFER, FAST, NARROW>, CH, bytes);
         if (e != cudaSuccess) return e;
         resident[dev] = nb > 0 ? nb : 1;
     }
     const int grid = persistent_grid(cx, resident[dev]);
-    launch_chained(g2p_kernel<CH, DEFER, FAST>, grid, CH, bytes, cx.stream, cx.scenes, cx.st, cx.st2, cx.ws, dt,
+    launch_chained(g2p_kernel<CH, DEFER, FAST, NARROW>, grid, CH, bytes, cx.stream, cx.scenes, cx.st, cx.st2, cx.ws, dt,
                    cx.status);
     return cudaGetLastError();
 }
@@ -724,8 +727,8 @@ cudaError_t launch_p2g(const Ctx &cx, float dt) {
     // blocks when there are more blocks than CTAs
     int grid = (int)(cx.total_blocks < (int64_t)cx.num_sms * 24 ? cx.total_blocks : (int64_t)cx.num_sms * 24);
     if (grid < 1) grid = 1;
-    launch_chained(p2g_kernel, grid, kP2GWarps * 32, bytes, cx.stream, cx.scenes, cx.n_scenes, cx.st, cx.ws, dt,
-                   cx.status);
+    launch_chained(cx.st.wide ? p2g_kernel<false> : p2g_kernel<true>, grid, kP2GWarps * 32, bytes, cx.stream, cx.scenes,
+                   cx.n_scenes, cx.st, cx.ws, dt, cx.status);
     return cudaGetLastError();
 }
 
@@ -744,22 +747,24 @@ cudaError_t launch_advance_colliders(MpmScene *scenes, int n_scenes, float time,
     return cudaGetLastError();
 }
 
-template <bool DEFER, bool FAST>
+template <bool DEFER, bool FAST, bool NARROW>
 static cudaError_t g2p_sized(const Ctx &cx, float dt) {
     switch (cx.ws.chunk_size) {
-        case 32: return g2p_t<32, DEFER, FAST>(cx, dt);
-        case 64: return g2p_t<64, DEFER, FAST>(cx, dt);
-        case 128: return g2p_t<128, DEFER, FAST>(cx, dt);
-        case 256: return g2p_t<256, DEFER, FAST>(cx, dt);
+        case 32: return g2p_t<32, DEFER, FAST, NARROW>(cx, dt);
+        case 64: return g2p_t<64, DEFER, FAST, NARROW>(cx, dt);
+        case 128: return g2p_t<128, DEFER, FAST, NARROW>(cx, dt);
+        case 256: return g2p_t<256, DEFER, FAST, NARROW>(cx, dt);
         default: return cudaErrorInvalidValue;
     }
 }
 
 cudaError_t launch_g2p(const Ctx &cx, float dt, G2PForm form) {
+    if (!cx.st2.wide)
+        return form == G2PForm::kDeferStress ? g2p_sized<true, false, true>(cx, dt) : g2p_sized<false, false, true>(cx, dt);
     switch (form) {
-        case G2PForm::kFast: return g2p_sized<false, true>(cx, dt);
-        case G2PForm::kDeferStress: return g2p_sized<true, true>(cx, dt);
-        default: return g2p_sized<false, false>(cx, dt);
+        case G2PForm::kFast: return g2p_sized<false, true, false>(cx, dt);
+        case G2PForm::kDeferStress: return g2p_sized<true, true, false>(cx, dt);
+        default: return g2p_sized<false, false, false>(cx, dt);
     }
 }
 
