@@ -107,12 +107,26 @@ __global__ void __launch_bounds__(kScanThreads) bucket_sums_kernel(Ws ws) {
     if (threadIdx.x == 0) ws.tile_sums[blockIdx.x] = t;
 }
 
+// Sums of kSuperTiles tile sums each, for grids of so many buckets that a CTA's sum over
+// all earlier tiles counts (it grows with the square of the buckets).  A group's three sums
+// go into the unused fourth words of its first three tile sums; nobody needs those of a
+// last group that has fewer.
+constexpr int kSuperTiles = kScanThreads;
+__global__ void __launch_bounds__(kScanThreads) super_sums_kernel(Ws ws, int n_tiles) {
+    chain_wait();
+    __shared__ int4 wsum[kScanWarps];
+    const int i = blockIdx.x * kSuperTiles + (int)threadIdx.x;
+    int4 v = i < n_tiles ? ws.tile_sums[i] : make_int4(0, 0, 0, 0);
+    const int4 t = cta_sum4(v, wsum);
+    if (threadIdx.x < 3 && i < n_tiles) ws.tile_sums[i].w = threadIdx.x == 0 ? t.x : (threadIdx.x == 1 ? t.y : t.z);
+}
+
 // Bucket offsets / cursors, the G2P chunk list and the P2G block list.  A CTA
 // owns KB buckets and finds what lies before them by itself, so no
 // CTA waits for another and no pass over tile sums comes in between: from the
 // counts of all earlier buckets (SUMS false: a few independent loads a thread
-// while there are at most kDirectBuckets of them), or from bucket_sums_kernel's
-// sums.  Then its warps take its non-empty buckets and write the 64 cell
+// while there are at most kDirectBuckets of them), from bucket_sums_kernel's
+// sums, or (past kSuperBuckets) from super_sums_kernel's first.  Then its warps take its non-empty buckets and write the 64 cell
 // offsets of each with a warp scan (two cells per lane), and its chunk-list
 // entries with one lane per chunk.  The last CTA publishes the list lengths.
 // (A kernel that scanned all tile sums behind an atomic ticket cost 5 to 12 us a
@@ -125,7 +139,10 @@ constexpr int kDirectBuckets = 8192;  // an 80^3 grid: up to eight 16-byte loads
 // CTAs enough, and each one's sum over the tile sums counts (256 instead of 64:
 // 64 scenes, 420k buckets, 74 -> 62 us).
 constexpr int kWideBuckets = 1 << 17;
-template <bool SUMS, int KB>
+// Past kSuperBuckets that sum is what counts: sort of a 512^3 grid (2.1M buckets) 121 us
+// with one level of sums, 119 with two; 800^3 441, 364; 1024^3 1,078, 692; 1280^3 2,809, 1,275.
+constexpr int kSuperBuckets = 1 << 20;
+template <int SUMS, int KB>  // SUMS: levels of sums to read (0-2)
 __global__ void __launch_bounds__(kScanThreads) scan_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
                                                             Ws ws) {
     chain_wait();
@@ -140,9 +157,18 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const MpmScene *__re
     // what lies before the CTA's buckets (b0 is a multiple of four, and no bucket
     // before it is the sentinel, the last one)
     int4 pre = make_int4(0, 0, 0, 0);
-    if (SUMS) {
+    if (SUMS > 0) {
         const int full = b0 / kSumTile;
-        for (int t = threadIdx.x; t < full; t += kScanThreads) pre = add4(pre, ws.tile_sums[t]);
+        int first = 0;  // tile
+        if (SUMS > 1) {
+            const int groups = full / kSuperTiles;
+            for (int g = threadIdx.x; g < groups; g += kScanThreads) {
+                const int4 *s = ws.tile_sums + (int64_t)g * kSuperTiles;
+                pre = add4(pre, make_int4(s[0].w, s[1].w, s[2].w, 0));
+            }
+            first = groups * kSuperTiles;
+        }
+        for (int t = first + (int)threadIdx.x; t < full; t += kScanThreads) pre = add4(pre, ws.tile_sums[t]);
         for (int h = full * kSumTile + (int)threadIdx.x; h < b0; h += kScanThreads)
             pre = add4(pre, bucket_triple(ws, h, ws.counts[h]));
     } else {
@@ -283,16 +309,20 @@ cudaError_t launch_keys(const Ctx &cx) {
 cudaError_t launch_sort(const Ctx &cx) {
     const int nbk = cx.ws.nbk;
     if (nbk <= kDirectBuckets) {
-        launch_chained(scan_kernel<false, 64>, (nbk + 63) / 64, kScanThreads, 0, cx.stream, cx.scenes, cx.n_scenes,
+        launch_chained(scan_kernel<0, 64>, (nbk + 63) / 64, kScanThreads, 0, cx.stream, cx.scenes, cx.n_scenes,
                        cx.ws);
     } else {
-        launch_chained(bucket_sums_kernel, (nbk + kSumTile - 1) / kSumTile, kScanThreads, 0, cx.stream, cx.ws);
+        const int n_tiles = (nbk + kSumTile - 1) / kSumTile;
+        launch_chained(bucket_sums_kernel, n_tiles, kScanThreads, 0, cx.stream, cx.ws);
+        if (nbk > kSuperBuckets)
+            launch_chained(super_sums_kernel, (n_tiles + kSuperTiles - 1) / kSuperTiles, kScanThreads, 0, cx.stream,
+                           cx.ws, n_tiles);
         if (nbk <= kWideBuckets)
-            launch_chained(scan_kernel<true, 64>, (nbk + 63) / 64, kScanThreads, 0, cx.stream, cx.scenes,
+            launch_chained(scan_kernel<1, 64>, (nbk + 63) / 64, kScanThreads, 0, cx.stream, cx.scenes,
                            cx.n_scenes, cx.ws);
         else
-            launch_chained(scan_kernel<true, 256>, (nbk + 255) / 256, kScanThreads, 0, cx.stream, cx.scenes,
-                           cx.n_scenes, cx.ws);
+            launch_chained(nbk > kSuperBuckets ? scan_kernel<2, 256> : scan_kernel<1, 256>, (nbk + 255) / 256,
+                           kScanThreads, 0, cx.stream, cx.scenes, cx.n_scenes, cx.ws);
     }
     // kScatterPer keys a thread, but never fewer than two CTAs an SM: the blocks to
     // clear do not shrink with the particles (a few CTAs clearing a sparse scene's
