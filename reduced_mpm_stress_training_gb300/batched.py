@@ -10,7 +10,8 @@ graph.  Scenes may mix sand and metal, particle counts and grid sizes; they
 share dt.
 
 ``autotune`` picks the G2P chunk size (particles per CTA) for a workload by
-timing the candidates, and caches the choice per device and workload shape.
+timing the candidates, and caches the choice per device, workload shape and build of
+the library.
 """
 from __future__ import annotations
 
@@ -95,10 +96,13 @@ def _cache_path() -> str:
 
 
 def workload_key(scenes: list[Scene], device) -> str:
+    """The device, the scenes' sizes and materials, and the library whose kernels were timed."""
     name = torch.cuda.get_device_name(device)
     shape = [(s.n_particles, s.n_grid, s.material) for s in scenes]
     h = hashlib.sha1(json.dumps(shape).encode()).hexdigest()[:16]
-    return f"{name}|{len(scenes)}|{sum(s.n_particles for s in scenes)}|{h}"
+    with open(A.lib_path(), "rb") as f:
+        build = hashlib.sha1(f.read()).hexdigest()[:16]
+    return f"{name}|{len(scenes)}|{sum(s.n_particles for s in scenes)}|{h}|{build}"
 
 
 def time_chunk_size(scenes: list[Scene], chunk: int, device, steps: int = 8) -> float:
