@@ -1,6 +1,9 @@
-// Device core of the tcgen05 network forward, shared by the standalone
-// forward (mpm_mlp_tc.cu) and the in-step surrogate stage (mpm_surrogate.cu).
-// See mpm_mlp_tc.cu for the operand layout and the synchronisation scheme.
+// tcgen05 helpers (operand layout, descriptors, MMA, mbarrier, tensor-memory loads) of the
+// network's forward (mpm_mlp_tc.cu), its backward (mpm_mlp_bw_tc.cu) and the decoder
+// (mpm_decoder.cu), and the tile forward of the in-step surrogate stage
+// (mpm_surrogate.cu): one 128-row tile at a time on 256 threads, two CTAs an SM.  The
+// standalone forward has its own pipelines; see there for the layout and the
+// synchronisation scheme.
 #pragma once
 
 #include "mpm_mlp.cuh"
@@ -123,25 +126,21 @@ __device__ __forceinline__ void stage_weights(TcSmem &s, const __nv_bfloat16 *w,
 }
 
 // bias + SiLU of 32 accumulator columns of this thread's row; writes the bf16
-// activations (columns c0..c0+31) into the A slabs and, if given, Z to zrow
-__device__ __forceinline__ void act_chunk(TcSmem &s, const float acc[32], const float *bias, int row, int c0,
-                                          __nv_bfloat16 *zrow) {
+// activations (columns c0..c0+31) into the A slabs
+__device__ __forceinline__ void act_chunk(TcSmem &s, const float acc[32], const float *bias, int row, int c0) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {  // 4 chunks of 8 columns = 16 bytes
-        uint32_t hv[4], zv[4];
+        uint32_t hv[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int c = q * 8 + 2 * e;
             const float z0 = acc[c] + bias[c0 + c], z1 = acc[c + 1] + bias[c0 + c + 1];
-            zv[e] = pack_bf16(z0, z1);
             hv[e] = pack_bf16(silu(z0), silu(z1));
         }
         const int k8 = (c0 >> 3) + q;
         *reinterpret_cast<uint4 *>(s.h + chunk_off(row, k8, kSlab)) = make_uint4(hv[0], hv[1], hv[2], hv[3]);
-        if (zrow) *reinterpret_cast<uint4 *>(zrow + c0 + q * 8) = make_uint4(zv[0], zv[1], zv[2], zv[3]);
     }
 }
-
 
 // CTA set-up: weights into the K-major layout, mbarrier, 128 TMEM columns.
 // All 128 threads call it; returns the TMEM base address.
@@ -194,11 +193,9 @@ __device__ __forceinline__ void tc_store_inputs(TcSmem &s, const float v[12]) {
 // The four layers on the 128-row tile whose inputs are in s.x.  Threads t and
 // t + 128 share row t (TMEM lanes are reachable from warps w and w + 4) and
 // take columns 0-63 and 64-127 of the hidden layers.  Thread t < 128 gets row
-// t's 16 (padded) outputs, bias added, in out; with z != null the bf16
-// pre-activations of layer l go to z[l] (row pointers, null for padding
-// rows).  Returns false (uniformly) on a timed-out wait.
-__device__ __forceinline__ bool tc_tile_forward(TcSmem &s, uint32_t tbase, uint32_t &phase, float out[16],
-                                                __nv_bfloat16 *const z[3]) {
+// t's 16 (padded) outputs, bias added, in out.  Returns false (uniformly) on a
+// timed-out wait.
+__device__ __forceinline__ bool tc_tile_forward(TcSmem &s, uint32_t tbase, uint32_t &phase, float out[16]) {
     const int tid = threadIdx.x, warp = tid >> 5;
     const int row = tid & (kRows - 1), half = tid >> 7;
     const uint32_t tlane = tbase + ((uint32_t)((warp & 3) * 32) << 16);
@@ -232,7 +229,7 @@ __device__ __forceinline__ bool tc_tile_forward(TcSmem &s, uint32_t tbase, uint3
             for (int c0 = half * (H / 2); c0 < (half + 1) * (H / 2); c0 += 32) {
                 float acc[32];
                 tmem_ld32(tlane + (uint32_t)c0, acc);
-                act_chunk(s, acc, s.bias + layer * H, row, c0, z ? z[layer] : nullptr);
+                act_chunk(s, acc, s.bias + layer * H, row, c0);
             }
         } else {
             float acc[32];

@@ -376,9 +376,9 @@ __global__ void __launch_bounds__(kSurWarps * 32, 1)
     }
 }
 
-// The in-step stage on the tcgen05 tensor cores: one CTA of 128 threads walks
-// the G2P chunk list in tiles of up to 128 particles of one scene (thread =
-// particle), runs the exact pre-pass, and -- if any particle of the tile
+// The in-step stage on the tcgen05 tensor cores: one CTA of 256 threads walks
+// the G2P chunk list in tiles of up to 128 particles of one scene (each of the
+// first 128 threads has one), runs the exact pre-pass, and -- if any particle of the tile
 // needs it -- the network on the tile (mpm_mlp_tc.cuh), then the correction
 // and gate.  A timed-out tensor-core wait raises MPM_ST_INTERNAL.
 constexpr int kTcRows = mlptc::kRows;
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(mlptc::kThreads, 2)
                     mlptc::tc_store_inputs(s, xi);
                 }
                 float out[16];
-                ok = mlptc::tc_tile_forward(s, tbase, phase, out, nullptr);
+                ok = mlptc::tc_tile_forward(s, tbase, phase, out);
                 if (!ok) break;
                 if (need) {
                     const float y6[6] = {out[0], out[1], out[2], out[3], out[4], out[5]};
@@ -523,8 +523,7 @@ cudaError_t launch_surrogate(const Ctx &cx, const void *mlp_params, const MpmSur
     int grid = (int)(items < 2 * (int64_t)cx.num_sms ? items : 2 * (int64_t)cx.num_sms);
     if (grid < 1) grid = 1;
     launch_chained(surrogate_tc_kernel, grid, mlptc::kThreads, bytes, cx.stream, cx.scenes, cx.st2, cx.ws, w, b, cfg,
-                   fallback, stats,
-                                                             cx.status);
+                   fallback, stats, cx.status);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     int fgrid = cx.num_sms * 4;
