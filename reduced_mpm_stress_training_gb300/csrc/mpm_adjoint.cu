@@ -342,11 +342,10 @@ __device__ __forceinline__ void load_F(const PState &st, int slot, float (&F)[9]
 // and spills at 2 blocks an SM -> 128 at 4: 82 -> 62 us at 131k particles (gather
 // unrolled 64; 168 registers at 3 blocks 65; 96 at 5, 72; blocks of 64 threads 64).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads, 4) g2p_adjoint_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
-                                                          PState st, Ws ws, const float *__restrict__ adj_out,
-                                                          float *__restrict__ adj_in,
-                                                          float4 *__restrict__ grid_adj, double *__restrict__ thb_out,
-                                                          float dt, bool vec) {
+__global__ void __launch_bounds__(kThreads, 4)
+    g2p_adjoint_kernel(const MpmScene *__restrict__ scenes, int n_scenes, PState st, Ws ws,
+                       const float *__restrict__ adj_out, float *__restrict__ adj_in, float4 *__restrict__ grid_adj,
+                       double *__restrict__ thb_out, float dt, bool vec) {
     chain_wait();
     float thb[3] = {0.0f, 0.0f, 0.0f};
     for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < ws.n; pos += gridDim.x * blockDim.x) {
@@ -574,9 +573,9 @@ __global__ void __launch_bounds__(256) grid_adjoint_kernel(const MpmScene *__res
 // and 4 words a particle where single words were 27: 33 -> 25 us at 131k
 // particles (128 registers at 4 blocks an SM: the same, with spills).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads, 3) p2g_adjoint_kernel(const MpmScene *__restrict__ scenes, int n_scenes,
-                                                          PState st, Ws ws, const float4 *__restrict__ grid_adj,
-                                                          float *__restrict__ adj_in, float dt, bool vec) {
+__global__ void __launch_bounds__(kThreads, 3)
+    p2g_adjoint_kernel(const MpmScene *__restrict__ scenes, int n_scenes, PState st, Ws ws,
+                       const float4 *__restrict__ grid_adj, float *__restrict__ adj_in, float dt, bool vec) {
     chain_wait();
     for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < ws.n; pos += gridDim.x * blockDim.x) {
         const int slot = ws.order[pos];
@@ -715,14 +714,11 @@ cudaError_t launch_adjoint(const Ctx &cx, const float *adj_out, float *adj_in, f
     const bool vec = ((reinterpret_cast<uintptr_t>(adj_out) | reinterpret_cast<uintptr_t>(adj_in)) & 15) == 0;
     launch_chained(zero_active_kernel, cx.num_sms * 4, 256, 0, cx.stream, cx.ws, grid_adj);
     launch_chained(g2p_adjoint_kernel, pgrid, kThreads, 0, cx.stream, cx.scenes, cx.n_scenes, cx.st, cx.ws, adj_out,
-                   adj_in,
-                                                     grid_adj, thb, dt, vec);
+                   adj_in, grid_adj, thb, dt, vec);
     launch_chained(grid_adjoint_kernel, ggrid > 0 ? ggrid : 1, 256, 0, cx.stream, cx.scenes, cx.n_scenes, cx.ws,
-                   grid_adj,
-                                                                      time, dt);
+                   grid_adj, time, dt);
     launch_chained(p2g_adjoint_kernel, pgrid, kThreads, 0, cx.stream, cx.scenes, cx.n_scenes, cx.st, cx.ws, grid_adj,
-                   adj_in, dt,
-                                                        vec);
+                   adj_in, dt, vec);
     return cudaGetLastError();
 }
 

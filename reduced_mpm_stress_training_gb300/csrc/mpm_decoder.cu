@@ -430,10 +430,9 @@ __device__ __forceinline__ bool pipe_and(int pipe, bool v) {
 }  // namespace dtc
 
 template <int P, bool NARROW>
-__global__ void __launch_bounds__(P * dtc::kRows, P == 2 ? 3 : 4) decoder_stress_tc_kernel(MpmStressDecoder d, PState st,
-                                                                          const float *__restrict__ label,
-                                                                          const float *__restrict__ mu, int n,
-                                                                          int *status) {
+__global__ void __launch_bounds__(P * dtc::kRows, P == 2 ? 3 : 4)
+    decoder_stress_tc_kernel(MpmStressDecoder d, PState st, const float *__restrict__ label,
+                             const float *__restrict__ mu, int n, int *status) {
     chain_wait();
     using namespace dtc;
     extern __shared__ __align__(128) unsigned char dtc_smem_raw[];

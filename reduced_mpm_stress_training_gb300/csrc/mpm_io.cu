@@ -303,8 +303,8 @@ cudaError_t launch_init_state(const Ctx &cx, const PState &other) {
 
 cudaError_t launch_load(const Ctx &cx, int field, const float *src) {
     if (cx.n == 0) return cudaSuccess;
-    launch_chained(load_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, field,
-                                                               field_components(field), src);
+    launch_chained(load_kernel, blocks_for(cx.n, 256), 256, 0, cx.stream, cx.st, cx.n, field, field_components(field),
+                   src);
     return cudaGetLastError();
 }
 

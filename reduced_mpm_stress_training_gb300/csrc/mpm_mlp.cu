@@ -361,8 +361,7 @@ int mpm_mlp_forward(const void *params, const float *x, float *y, const float *t
     FwdIO io{x, y, target, static_cast<__nv_bfloat16 *>(zsave), static_cast<__nv_bfloat16 *>(dy), loss,
              grad_scale, n};
     mpm::launch_chained(mlp_forward_kernel, mlp_grid((n + 15) / 16, 8, 1), 256, sizeof(WSmem),
-                        static_cast<cudaStream_t>(stream),
-        w, b, io);
+                        static_cast<cudaStream_t>(stream), w, b, io);
     return cudaGetLastError() == cudaSuccess ? MPM_OK : MPM_ERR_CUDA;
 }
 
@@ -414,8 +413,8 @@ int mpm_mlp_adam(float *master, float *m, float *v, const float *grad, void *par
     const float c2 = 1.0f / (1.0f - powf(beta2, (float)step));
     __nv_bfloat16 *wbf = static_cast<__nv_bfloat16 *>(params);
     float *bias = reinterpret_cast<float *>(static_cast<char *>(params) + (int64_t)W_COUNT * 2);
-    mpm::launch_chained(mlp_adam_kernel, (count + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream),
-        master, m, v, grad, wbf, bias, count, lr, beta1, beta2, eps, c1, c2);
+    mpm::launch_chained(mlp_adam_kernel, (count + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream), master, m, v,
+                        grad, wbf, bias, count, lr, beta1, beta2, eps, c1, c2);
     return cudaGetLastError() == cudaSuccess ? MPM_OK : MPM_ERR_CUDA;
 }
 

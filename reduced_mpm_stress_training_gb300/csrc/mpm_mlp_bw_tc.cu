@@ -422,8 +422,7 @@ cudaError_t launch_mlp_backward_tc(const void *params, const float *x, const voi
     // one CTA per SM (each holds all 512 tensor-memory columns)
     const int grid = (int)(tiles < (int64_t)num_sms ? tiles : (int64_t)num_sms);
     launch_chained(mlp_backward_tc_kernel, grid, kBwThreads, bytes, stream, w, x,
-                   static_cast<const __nv_bfloat16 *>(zsave),
-                                                              static_cast<const __nv_bfloat16 *>(dy), grad, n, err);
+                   static_cast<const __nv_bfloat16 *>(zsave), static_cast<const __nv_bfloat16 *>(dy), grad, n, err);
     return cudaGetLastError();
 }
 

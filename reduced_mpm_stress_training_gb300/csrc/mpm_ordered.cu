@@ -459,8 +459,7 @@ cudaError_t launch_p2g_ordered(const Ctx &cx, float dt, void *scratch) {
     // rest start as others finish, which balances blocks of unequal size
     const int64_t tw = cx.total_blocks < (int64_t)cx.num_sms * 32 ? cx.total_blocks : (int64_t)cx.num_sms * 32;
     launch_chained(p2g_tiles_kernel, (unsigned)(tw > 0 ? tw : 1), 32, 0, cx.stream, cx.scenes, cx.n_scenes, cx.st,
-                   cx.ws, dt,
-                                                                        cx.status, partials, blk_index);
+                   cx.ws, dt, cx.status, partials, blk_index);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int64_t want = (cx.total_blocks + 3) / 4;
     int grid = (int)(want < (int64_t)cx.num_sms * 8 ? want : (int64_t)cx.num_sms * 8);

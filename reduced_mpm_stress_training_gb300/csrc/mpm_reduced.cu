@@ -224,8 +224,7 @@ __global__ void __launch_bounds__(kRedWarps * 32) reduced_p2g_kernel(const MpmSc
         const float m = q0.w;
         const float ts = -__fdiv_rn(m, g.density[uid]) * dt * inv_dx;  // -(m / density) dt / dx, :395
         pay[warp][0][at] = make_float4(fx[0], fx[1], fx[2], m);
-        pay[warp][1][at] = make_float4(q2.w, q3.x, q3.y,
-                                         __int_as_float(key));
+        pay[warp][1][at] = make_float4(q2.w, q3.x, q3.y, __int_as_float(key));
         pay[warp][2][at] = make_float4(tau[0] * ts, tau[1] * ts, tau[2] * ts, tau[3] * ts);
         pay[warp][3][at] = make_float4(tau[4] * ts, tau[5] * ts, tau[6] * ts, tau[7] * ts);
         pay[warp][4][at] = make_float4(tau[8] * ts, 0.0f, 0.0f, 0.0f);
@@ -441,8 +440,8 @@ cudaError_t launch_p2g2p_reduced(const Ctx &cx, const MpmReducedGrid &g, float t
             launch_chained(mark_kernel<2>, (unsigned)((g.n_samples + 7) / 8), 256, 0, cx.stream, cx.scenes, cx.st,
                            cx.ws.slot_of_uid, g, g.neighboring_cells, cx.n, cx.status);
         launch_chained(cx.st.wide ? reduced_p2g_kernel<false> : reduced_p2g_kernel<true>,
-                       (cx.n + kRedWarps * 32 - 1) / (kRedWarps * 32), kRedWarps * 32, 0, cx.stream, cx.scenes, cx.st, g,
-                       cx.n, dt, cx.status);
+                       (cx.n + kRedWarps * 32 - 1) / (kRedWarps * 32), kRedWarps * 32, 0, cx.stream, cx.scenes,
+                       cx.st, g, cx.n, dt, cx.status);
     }
     const int64_t want = (nn + 255) / 256;
     const int blocks = (int)(want < (int64_t)cx.num_sms * 16 ? want : (int64_t)cx.num_sms * 16);

@@ -124,11 +124,12 @@ __global__ void __launch_bounds__(kScanThreads) super_sums_kernel(Ws ws, int n_t
 // Bucket offsets / cursors, the G2P chunk list and the P2G block list.  A CTA
 // owns KB buckets and finds what lies before them by itself, so no
 // CTA waits for another and no pass over tile sums comes in between: from the
-// counts of all earlier buckets (SUMS false: a few independent loads a thread
-// while there are at most kDirectBuckets of them), from bucket_sums_kernel's
-// sums, or (past kSuperBuckets) from super_sums_kernel's first.  Then its warps take its non-empty buckets and write the 64 cell
-// offsets of each with a warp scan (two cells per lane), and its chunk-list
-// entries with one lane per chunk.  The last CTA publishes the list lengths.
+// counts of all earlier buckets (a few independent loads a thread while there are
+// at most kDirectBuckets of them), from bucket_sums_kernel's sums, or (past
+// kSuperBuckets) from super_sums_kernel's first.  Then its warps take its
+// non-empty buckets and write the 64 cell offsets of each with a warp scan (two
+// cells per lane), and its chunk-list entries with one lane per chunk.  The last
+// CTA publishes the list lengths.
 // (A kernel that scanned all tile sums behind an atomic ticket cost 5 to 12 us a
 // substep.  Handing the ranges out with atomics, in the order CTAs arrive, is as
 // fast here but scatters neighbouring blocks: P2G 3 % slower on 64 scenes.)
@@ -301,8 +302,8 @@ __global__ void __launch_bounds__(256) scatter_kernel(PState st, Ws ws, int n) {
 
 cudaError_t launch_keys(const Ctx &cx) {
     if (cx.n == 0) return cudaSuccess;
-    launch_chained(key_kernel, (cx.n + 255) / 256, 256, 0, cx.stream, cx.scenes, cx.n_scenes, cx.st, cx.ws,
-                                                           cx.n, cx.status);
+    launch_chained(key_kernel, (cx.n + 255) / 256, 256, 0, cx.stream, cx.scenes, cx.n_scenes, cx.st, cx.ws, cx.n,
+                   cx.status);
     return cudaGetLastError();
 }
 

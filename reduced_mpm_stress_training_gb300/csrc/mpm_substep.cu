@@ -705,17 +705,17 @@ static cudaError_t g2p_t(const Ctx &cx, float dt) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    const auto kernel = g2p_kernel<CH, DEFER, FAST, NARROW>;
     if (resident[dev] == 0) {
-        e = cudaFuncSetAttribute(g2p_kernel<CH, DEFER, FAST, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return e;
         int nb = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, g2p_kernel<CH, DEFER, FAST, NARROW>, CH, bytes);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, CH, bytes);
         if (e != cudaSuccess) return e;
         resident[dev] = nb > 0 ? nb : 1;
     }
     const int grid = persistent_grid(cx, resident[dev]);
-    launch_chained(g2p_kernel<CH, DEFER, FAST, NARROW>, grid, CH, bytes, cx.stream, cx.scenes, cx.st, cx.st2, cx.ws, dt,
-                   cx.status);
+    launch_chained(kernel, grid, CH, bytes, cx.stream, cx.scenes, cx.st, cx.st2, cx.ws, dt, cx.status);
     return cudaGetLastError();
 }
 
@@ -759,8 +759,9 @@ static cudaError_t g2p_sized(const Ctx &cx, float dt) {
 }
 
 cudaError_t launch_g2p(const Ctx &cx, float dt, G2PForm form) {
-    if (!cx.st2.wide)
-        return form == G2PForm::kDeferStress ? g2p_sized<true, false, true>(cx, dt) : g2p_sized<false, false, true>(cx, dt);
+    if (!cx.st2.wide)  // one form for each result
+        return form == G2PForm::kDeferStress ? g2p_sized<true, false, true>(cx, dt)
+                                             : g2p_sized<false, false, true>(cx, dt);
     switch (form) {
         case G2PForm::kFast: return g2p_sized<false, true, false>(cx, dt);
         case G2PForm::kDeferStress: return g2p_sized<true, true, false>(cx, dt);
