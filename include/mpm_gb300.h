@@ -240,8 +240,7 @@ int mpm_p2g2p(MpmBuffers *b, float time, float dt, void *stream);
 
 /* The substep's stages, for callers that interleave their own work and for
  * per-stage checks.  mpm_p2g2p == sort, p2g, grid_update, g2p up to float32
- * rounding: it runs its own compilation of the last stage, while mpm_g2p keeps
- * one whose float32 results stay the same bit for bit. */
+ * rounding: it runs its own compilation of the last stage. */
 int mpm_sort(MpmBuffers *b, void *stream); /* block keys, counting sort, re-sort */
 int mpm_p2g(MpmBuffers *b, float dt, void *stream); /* mpm_utils.py:190-227 */
 int mpm_grid_update(MpmBuffers *b, float time, float dt, void *stream); /* :229-237 + colliders */

@@ -430,7 +430,7 @@ int mpm_grid_update(MpmBuffers *b, float time, float dt, void *stream) {
 int mpm_g2p(MpmBuffers *b, float dt, void *stream) {
     NvtxRange nvtx_("mpm_g2p");
     if (!buffers_ok(b)) return MPM_ERR_ARG;
-    MPM_CHECK(mpm::launch_g2p(make_ctx(b, stream, b->cur), dt, mpm::G2PForm::kPinned));
+    MPM_CHECK(mpm::launch_g2p(make_ctx(b, stream, b->cur), dt, mpm::G2PForm::kStage));
     b->cur ^= 1;  // G2P wrote the sorted, updated records into the other buffer
     b->substep += 1;
     return MPM_OK;

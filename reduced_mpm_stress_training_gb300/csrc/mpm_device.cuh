@@ -86,8 +86,8 @@ __device__ __forceinline__ float &recword(const PState &st, int slot, int w) {
     return reinterpret_cast<float *>(recq(st, slot, w >> 2))[w & 3];
 }
 
-// A kernel that launch_chained starts may be resident while the kernel before it
-// in the stream still runs: nothing is read or written before this returns (the
+// A kernel that launch_chained starts may be resident before the kernel before it in
+// the stream has completed: nothing is read or written before this returns (the
 // earlier kernel, and all before it, complete and visible).
 __device__ __forceinline__ void chain_wait() {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");

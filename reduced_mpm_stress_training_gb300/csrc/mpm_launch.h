@@ -33,12 +33,14 @@ cudaError_t launch_p2g(const Ctx &cx, float dt);
 int64_t ordered_scratch_bytes(int64_t total_blocks);
 cudaError_t launch_p2g_ordered(const Ctx &cx, float dt, void *scratch);
 // Starts a kernel whose first statement is chain_wait() (programmatic dependent
-// launch): its launch and its blocks' start overlap the tail of the kernel before it
-// in the stream, which saves the gap of about 2 us that an ordinary launch leaves
+// launch).  No kernel says launch_dependents, so the next one is launched once every
+// block of the one before it in the stream has exited: what overlaps is the launch
+// itself and the completion of the earlier kernel (its memory flush), and chain_wait
+// covers the rest.  That saves the gap of about 2 us that an ordinary launch leaves
 // (eager substep of 32k particles 39.1 -> 25.8 us, 300k 88.1 -> 74.2, 1M 178 -> 166;
 // in a graph, where the gaps are shorter, 26.6 -> 24.8, 75.0 -> 72.5, 164 -> 164).
-// No kernel says launch_dependents itself: blocks of the next kernel that wait for it
-// all the while take the place of its own, and P2G's next wave (32k in a graph 29.4).
+// With launch_dependents at each kernel's entry, waiting blocks of the next kernel take
+// the place of the running one's own, and of P2G's next wave (32k in a graph 29.4).
 template <class... P, class... A>
 cudaError_t launch_chained(void (*kernel)(P...), int64_t grid, int block, size_t smem, cudaStream_t stream,
                            A... args) {
@@ -56,10 +58,10 @@ cudaError_t launch_chained(void (*kernel)(P...), int64_t grid, int block, size_t
 }
 
 cudaError_t launch_grid(const Ctx &cx, float time, float dt);
-// kFast: the substep's form; kPinned: results that do not change from build to
-// build (the stage entry point and the ordered mode); kDeferStress: store
+// kFast: the substep's form; kStage: the one of the stage entry point and the ordered
+// mode (another compilation, see mpm_ordered.cu for why it stays); kDeferStress: store
 // F_trial as F and skip the return map (surrogate stage follows)
-enum class G2PForm { kFast, kPinned, kDeferStress };
+enum class G2PForm { kFast, kStage, kDeferStress };
 cudaError_t launch_g2p(const Ctx &cx, float dt, G2PForm form);
 
 // surrogate stress stage (mpm_surrogate.cu): network stress with exact-invariant

@@ -460,10 +460,10 @@ __device__ __forceinline__ int g2p_slot(const Ws &ws, const int4 &ch) {
 // stage): F_trial is stored as F and the stress words are zeroed.
 // NARROW: `out` is a buffer of 16-byte alignment (see ldpair).
 // FAST: the form that mpm_p2g2p runs (on buffers that take 32-byte accesses), with five
-// 128-thread CTAs per SM (96 registers) instead of four and less integer work.  The mpm_g2p stage and the
-// ordered mode run the other form: ptxas fuses multiplies and adds differently
-// under another register budget, and they promise float32 results that stay
-// the same bit for bit (see mpm_ordered.cu).
+// 128-thread CTAs per SM (96 registers) instead of four and less integer work.  The mpm_g2p
+// stage and the ordered mode run the other form: ptxas fuses multiplies and adds
+// differently under another register budget, and the ordered mode keeps its roundings
+// (see mpm_ordered.cu).
 template <int CH, bool DEFER, bool FAST, bool NARROW>
 __global__ void __launch_bounds__(CH, FAST ? 640 / CH : 0) g2p_kernel(const MpmScene *__restrict__ scenes, PState st,
                                                  PState out, Ws ws, float dt, int *status) {
