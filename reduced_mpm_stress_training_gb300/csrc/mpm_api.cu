@@ -427,14 +427,16 @@ int mpm_grid_update(MpmBuffers *b, float time, float dt, void *stream) {
     return MPM_OK;
 }
 
-int mpm_g2p(MpmBuffers *b, float dt, void *stream) {
+static int run_g2p(MpmBuffers *b, float dt, void *stream, mpm::G2PForm form) {
     NvtxRange nvtx_("mpm_g2p");
     if (!buffers_ok(b)) return MPM_ERR_ARG;
-    MPM_CHECK(mpm::launch_g2p(make_ctx(b, stream, b->cur), dt, mpm::G2PForm::kStage));
+    MPM_CHECK(mpm::launch_g2p(make_ctx(b, stream, b->cur), dt, form));
     b->cur ^= 1;  // G2P wrote the sorted, updated records into the other buffer
     b->substep += 1;
     return MPM_OK;
 }
+
+int mpm_g2p(MpmBuffers *b, float dt, void *stream) { return run_g2p(b, dt, stream, mpm::G2PForm::kStage); }
 
 int64_t mpm_p2g_ordered_bytes(const MpmPlan *plan) {
     if (!plan || plan->total_blocks < 0) return -1;
@@ -463,10 +465,7 @@ int mpm_p2g2p(MpmBuffers *b, float time, float dt, void *stream) {
     if (r) return r;
     if ((r = mpm_p2g(b, dt, stream))) return r;
     if ((r = mpm_grid_update(b, time, dt, stream))) return r;
-    MPM_CHECK(mpm::launch_g2p(make_ctx(b, stream, b->cur), dt, mpm::G2PForm::kFast));
-    b->cur ^= 1;  // as mpm_g2p
-    b->substep += 1;
-    return MPM_OK;
+    return run_g2p(b, dt, stream, mpm::G2PForm::kFast);
 }
 
 static bool surrogate_cfg_ok(const MpmSurrogateConfig *c) {
