@@ -334,13 +334,13 @@ __device__ __forceinline__ void load_F(const PState &st, int slot, float (&F)[9]
 
 // ---------------------------------------------------------------------------
 // G2P adjoint: thread per sorted position.  Bound by instruction issue and
-// fetch at few warps an SM (28 M instructions, 46 % of the issue slots; DRAM 7 %),
+// fetch at few warps an SM (30 M instructions, 55 % of the issue slots; DRAM 8 %),
 // so the code and the registers were cut: both node loops run a plane at a time
 // (27 copies of each body waited for instructions), the scatter reads the
 // velocities again instead of holding 81 registers since the gather, and F, the
 // position and the weights are made again after the return map.  255 registers
-// and spills at 2 blocks an SM -> 128 at 4: 82 -> 62 us at 131k particles (gather
-// unrolled 64; 168 registers at 3 blocks 65; 96 at 5, 72; blocks of 64 threads 64).
+// (68 bytes of spills) at 2 blocks an SM -> 128 (124 bytes) at 4: 82 -> 62 us at 131k
+// particles (gather unrolled 64; 168 registers at 3 blocks 65; 96 at 5, 72; blocks of 64 threads 64).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads, 4)
     g2p_adjoint_kernel(const MpmScene *__restrict__ scenes, int n_scenes, PState st, Ws ws,

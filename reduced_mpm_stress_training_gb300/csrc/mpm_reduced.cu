@@ -151,10 +151,11 @@ __device__ __forceinline__ bool stress_dp_spectral(const float F[9], float mu, f
 // (i, j) sums its three z nodes in registers over consecutive particles of one
 // base cell and issues one 16-byte atomic per node when the cell changes.  The
 // records are in the cell order of the last substep and the particles have
-// moved since, so the warp first brings particles of one cell together: the
-// atomics (27 per run) are what bounds the kernel.  Measured on 1M marked
-// particles displaced by an eighth of a cell: 81 us; with
-// an SVD per stress and segmented shuffles over the runs as they lie, 126 us.
+// moved since, so the warp first brings particles of one cell together, for fewer
+// runs of 27 atomics.  Measured on 1M marked particles displaced by an eighth of a
+// cell: 82 us; with an SVD per stress and segmented shuffles over the runs as they
+// lie, 126 us.  64 M warp instructions at 66 % of the issue slots, DRAM 21 %: issue,
+// and the latency of the record, F_disp and density loads.
 constexpr int kRedWarps = 4;
 constexpr int kRedPay = 5;  // float4 of a particle's scatter data
 template <bool NARROW>
