@@ -556,8 +556,8 @@ class MPMEngine:
         self._status_stream.synchronize()
 
     def poll_status(self, wait: bool = False) -> int:
-        """Read the status word after the last substep (lazy; no sync
-        unless wait=True) and act on it per ``on_error``."""
+        """Read the status word after the last substep (lazy: unless wait=True, it
+        waits for the word's own copy at most) and act on it per ``on_error``."""
         if not self._pending:
             return 0
         if not wait and not self._status_event.query():
